@@ -167,7 +167,7 @@ __device__ __forceinline__ bool face_flux_with(PL pl, PR pr, SL sl, SR sr, doubl
   }
   // eos_p_cs (eos.f90:209-219) with erad = 0
   const double ptl0 = gm1 * eil, ptr0 = gm1 * eir;
-  const double csl = sqrt(dv.div(gamma * ptl0, dl, rdl)), csr = sqrt(dv.div(gamma * ptr0, dr, rdr));
+  const double csl = dv.root(dv.div(gamma * ptl0, dl, rdl)), csr = dv.root(dv.div(gamma * ptr0, dr, rdr));
   const double ptl = ptl0 + 0.5 * (b1l * b1l + b2l * b2l + b3l * b3l);
   const double ptr = ptr0 + 0.5 * (b1r * b1r + b2r * b2r + b3r * b3r);
   const double cfl = get_cf(dl, csl, b1l, b2l, b3l, dv, rdl);

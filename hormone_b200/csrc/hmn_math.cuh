@@ -24,14 +24,19 @@ template <typename T>
 __device__ __forceinline__ T fmax2(T a, T b) { return a > b ? a : b; }
 
 // Division policies: div(a, b, r) is a/b, where r = rec(b) was formed once
-// for every quotient with the denominator b.  PlainDiv divides (r is b
-// itself); FastDiv (hmn_div.cuh) forms RN(1/b) once and corrects each
-// quotient to RN(a/b), flagging operands it cannot take.
+// for every quotient with the denominator b, and root(x) is sqrt(x).
+// PlainDiv divides (r is b itself); FastDiv (hmn_div.cuh) forms RN(1/b) once
+// and corrects each quotient to RN(a/b), flagging operands it cannot take.
+// FastDiv takes positive denominators only, so expressions are written with
+// the positive one of b and -b (negating both operands changes no bit of the
+// quotient).
 struct PlainDiv {
   template <typename T>
   __device__ __forceinline__ T rec(T b) { return b; }
   template <typename T>
   __device__ __forceinline__ T div(T a, T b, T) { return a / b; }
+  template <typename T>
+  __device__ __forceinline__ T root(T x) { return sqrt(x); }
 };
 
 // Generalised minmod with theta = 1.4 on inverse spacings (fluxlimiter.f90:40-56).
@@ -107,7 +112,7 @@ __device__ __forceinline__ T get_cf(T d, T cs, T b1, T b2, T b3, D& dv, T rd) {
   T bb3 = dv.div(b3 * b3, d, rd);
   T bbsq = bb1 + bb2 + bb3;
   T t = asq + bbsq;
-  return sqrt(T(0.5) * (t + sqrt(t * t - T(4.0) * asq * bb1)));
+  return dv.root(T(0.5) * (t + dv.root(t * t - T(4.0) * asq * bb1)));
 }
 template <typename T>
 __device__ __forceinline__ T get_cf(T d, T cs, T b1, T b2, T b3) {
@@ -139,11 +144,11 @@ __device__ __forceinline__ void hlld(T f[9], T cfl, T cfr, T v1l, T v1r, T v2l, 
   const T den = wr * dr - wl * dl;
   const T rden = dvp.rec(den);
   const T sm = dvp.div(wr * dr * v1r - wl * dl * v1l - ptr + ptl, den, rden);
-  const T slsm = sl - sm, srsm = sr - sm;
-  const T rslsm = dvp.rec(slsm), rsrsm = dvp.rec(srsm);
-  const T dla0 = dvp.div(dl * wl, slsm, rslsm);
+  const T smsl = sm - sl, srsm = sr - sm;  // both positive
+  const T rsmsl = dvp.rec(smsl), rsrsm = dvp.rec(srsm);
+  const T dla0 = dvp.div(-(dl * wl), smsl, rsmsl);
   const T dra0 = dvp.div(dr * wr, srsm, rsrsm);
-  const T sqla = sqrt(dla0), sqra = sqrt(dra0);
+  const T sqla = dvp.root(dla0), sqra = dvp.root(dra0);
   const T sla = sm - dvp.div(fabs(b1), sqla, dvp.rec(sqla));
   const T sra = sm + dvp.div(fabs(b1), sqra, dvp.rec(sqra));
   const T pta = dvp.div(wr * dr * ptl - wl * dl * ptr + dl * dr * wr * wl * (v1r - v1l), den, rden);
@@ -161,9 +166,9 @@ __device__ __forceinline__ void hlld(T f[9], T cfl, T cfr, T v1l, T v1r, T v2l, 
   const T b2ra = dvp.div(b2r * numr, denr, rdenr);
   const T b3la = dvp.div(b3l * numl, denl, rdenl);
   const T b3ra = dvp.div(b3r * numr, denr, rdenr);
-  const T ela = dvp.div(wl * el - ptl * v1l + pta * sm +
-                           b1 * ((v1l * b1 + v2l * b2l + v3l * b3l) - (sm * b1 + v2la * b2la + v3la * b3la)),
-                       slsm, rslsm);
+  const T ela = dvp.div(-(wl * el - ptl * v1l + pta * sm +
+                           b1 * ((v1l * b1 + v2l * b2l + v3l * b3l) - (sm * b1 + v2la * b2la + v3la * b3la))),
+                       smsl, rsmsl);
   const T era = dvp.div(wr * er - ptr * v1r + pta * sm +
                            b1 * ((v1r * b1 + v2r * b2r + v3r * b3r) - (sm * b1 + v2ra * b2ra + v3ra * b3ra)),
                        srsm, rsrsm);
@@ -172,7 +177,7 @@ __device__ __forceinline__ void hlld(T f[9], T cfl, T cfr, T v1l, T v1r, T v2l, 
   const T rsqsum = dvp.rec(sqsum);
   const T v2aa = dvp.div(sqla * v2la + sqra * v2ra + (b2ra - b2la) * s1, sqsum, rsqsum);
   const T v3aa = dvp.div(sqla * v3la + sqra * v3ra + (b3ra - b3la) * s1, sqsum, rsqsum);
-  const T sqlr = sqrt(dla0 * dra0);
+  const T sqlr = dvp.root(dla0 * dra0);
   const T b2aa = dvp.div(sqla * b2ra + sqra * b2la + sqlr * (v2ra - v2la) * s1, sqsum, rsqsum);
   const T b3aa = dvp.div(sqla * b3ra + sqra * b3la + sqlr * (v3ra - v3la) * s1, sqsum, rsqsum);
   const T vbaa = v2aa * b2aa + v3aa * b3aa;
