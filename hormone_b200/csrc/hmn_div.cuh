@@ -56,9 +56,16 @@ __device__ __forceinline__ bool fin_range(double x) {
   return t - (523u << 21) < (1001u << 21);
 }
 
-// x in [2^-500, 2^501) and positive (a sign bit makes the difference large)
+// x in [2^LO, 2^HI) and positive (a sign bit makes the difference large)
+template <int LO = -500, int HI = 501>
 __device__ __forceinline__ bool pos_range(double x) {
-  return (unsigned)__double2hiint(x) - (523u << 20) < (1001u << 20);
+  return (unsigned)__double2hiint(x) - ((unsigned)(1023 + LO) << 20) < ((unsigned)(HI - LO) << 20);
+}
+
+// |x| below 2^HI (infinities and NaN are not)
+template <int HI>
+__device__ __forceinline__ bool below(double x) {
+  return ((unsigned)__double2hiint(x) & 0x7fffffffu) < ((unsigned)(1023 + HI) << 20);
 }
 
 __device__ __forceinline__ bool is_zero(double x) {
@@ -85,19 +92,23 @@ __device__ __forceinline__ double rsqrt_approx(double x) {
   return y;
 }
 
-// 1/b within about one ulp, without branches (the third-order step above);
-// for the mixed-precision form, which is not bound to IEEE quotients.  A zero
-// b gives NaN where IEEE gives infinity.
+// 1/b within about one ulp, without branches (two Newton-Raphson steps from
+// the approximation); for the mixed-precision form, which is not bound to
+// IEEE quotients.  A zero b gives NaN where IEEE gives infinity.
 __device__ __forceinline__ double rcp_nr(double b) {
-  const double y = rcp_approx(b);
-  const double e = __fma_rn(-b, y, 1.0);
-  return __fma_rn(y, __fma_rn(e, e, e), y);
+  double y = rcp_approx(b);
+  double e = __fma_rn(-b, y, 1.0);
+  y = __fma_rn(y, e, y);
+  e = __fma_rn(-b, y, 1.0);
+  return __fma_rn(y, e, y);
 }
 
 // RN(1/b) of a b that the caller has checked
 __device__ __forceinline__ double recip_core(double b) {
-  const double y = rcp_nr(b);  // within one ulp of 1/b
-  const double e = __fma_rn(-b, y, 1.0);
+  double y = rcp_approx(b);
+  double e = __fma_rn(-b, y, 1.0);
+  y = __fma_rn(y, __fma_rn(e, e, e), y);  // within one ulp of 1/b
+  e = __fma_rn(-b, y, 1.0);
   return __fma_rn(y, e, y);
 }
 
@@ -157,7 +168,13 @@ __device__ __forceinline__ double sqrt_pos(double x, bool& bad) {
 // 256^3 8.13 -> 7.10 ms, 97x75x62 box 17.3 -> 15.3 ms for 16 steps, 48 KH
 // boxes 76.5 -> 67.6 ms for 16 steps, a tube's step chain 6 % shorter.
 struct FastDiv {
+  static constexpr bool flags = true;  // results may be refused
   bool bad = false;
+  // what the hydrodynamic flux asks of its operands beyond the above
+  template <int LO, int HI>
+  __device__ __forceinline__ void need_pos(double x) { bad = bad | !pos_range<LO, HI>(x); }
+  template <int HI>
+  __device__ __forceinline__ void need_below(double x) { bad = bad | !below<HI>(x); }
   __device__ __forceinline__ double rec(double b) { return recip_pos(b, bad); }
   __device__ __forceinline__ double div(double a, double b, double y) { return div_pos(a, b, y, bad); }
   __device__ __forceinline__ double root(double x) { return sqrt_pos(x, bad); }

@@ -168,6 +168,18 @@ __device__ __forceinline__ bool face_flux_with(PL pl, PR pr, SL sl, SR sr, doubl
   // eos_p_cs (eos.f90:209-219) with erad = 0
   const double ptl0 = gm1 * eil, ptr0 = gm1 * eir;
   const double csl = dv.root(dv.div(gamma * ptl0, dl, rdl)), csr = dv.root(dv.div(gamma * ptr0, dr, rdr));
+  if constexpr (!MAG && D::flags) {  // the policy that recomputes what it refuses with the full solver
+    dv.template need_pos<-150, 200>(dl);
+    dv.template need_pos<-150, 200>(dr);
+    dv.template need_below<150>(v1l);
+    dv.template need_below<150>(v1r);
+    dv.template need_below<150>(v2l);
+    dv.template need_below<150>(v2r);
+    dv.template need_below<150>(v3l);
+    dv.template need_below<150>(v3r);
+    hllc(fl, csl, csr, v1l, v1r, v2l, v2r, v3l, v3r, dl, dr, el, er, ptl0, ptr0, dv);
+    return true;
+  }
   const double ptl = ptl0 + 0.5 * (b1l * b1l + b2l * b2l + b3l * b3l);
   const double ptr = ptr0 + 0.5 * (b1r * b1r + b2r * b2r + b3r * b3r);
   const double cfl = get_cf(dl, csl, b1l, b2l, b3l, dv, rdl);

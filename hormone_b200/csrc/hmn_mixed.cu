@@ -201,12 +201,18 @@ __device__ __forceinline__ void axis_pass_mixed(const GridDev& G, const StageArg
       const float b1lf = (float)b1l, b1rf = (float)b1r, b2lf = (float)b2l, b2rf = (float)b2r;
       const float b3lf = (float)b3l, b3rf = (float)b3r;
       const float csl = sqrtf(gam * ptl0 / dlf), csr = sqrtf(gam * ptr0 / drf);
-      const float ptl = ptl0 + 0.5f * (b1lf * b1lf + b2lf * b2lf + b3lf * b3lf);
-      const float ptr = ptr0 + 0.5f * (b1rf * b1rf + b2rf * b2rf + b3rf * b3rf);
-      const float cfl = get_cf(dlf, csl, b1lf, b2lf, b3lf);
-      const float cfr = get_cf(drf, csr, b1rf, b2rf, b3rf);
-      hlld<float>(fl, cfl, cfr, (float)v1l, (float)v1r, (float)v2l, (float)v2r, (float)v3l, (float)v3r, dlf, drf,
-                  (float)el, (float)er, ptl, ptr, b1lf, b1rf, b2lf, b2rf, b3lf, b3rf, (float)phil, (float)phir, ch);
+      if constexpr (!MAG) {  // no field: the star states of the contact wave only
+        PlainDiv dv;
+        hllc<float>(fl, csl, csr, (float)v1l, (float)v1r, (float)v2l, (float)v2r, (float)v3l, (float)v3r, dlf, drf,
+                    (float)el, (float)er, ptl0, ptr0, dv);
+      } else {
+        const float ptl = ptl0 + 0.5f * (b1lf * b1lf + b2lf * b2lf + b3lf * b3lf);
+        const float ptr = ptr0 + 0.5f * (b1rf * b1rf + b2rf * b2rf + b3rf * b3rf);
+        const float cfl = get_cf(dlf, csl, b1lf, b2lf, b3lf);
+        const float cfr = get_cf(drf, csr, b1rf, b2rf, b3rf);
+        hlld<float>(fl, cfl, cfr, (float)v1l, (float)v1r, (float)v2l, (float)v2r, (float)v3l, (float)v3r, dlf, drf,
+                    (float)el, (float)er, ptl, ptr, b1lf, b1rf, b2lf, b2rf, b3lf, b3rf, (float)phil, (float)phir, ch);
+      }
     }
     if (AX == 2 && G.fb != nullptr && t0[2] + f == 0) {  // boundary code 10 (fluxboundary.f90:42-87)
 #pragma unroll
