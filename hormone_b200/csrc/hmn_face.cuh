@@ -60,7 +60,7 @@ __device__ __forceinline__ void slopes_with(const double* pm, const double* p0, 
       eintl = eintl - 0.5 * (L[S_B] * L[S_B] + L[S_B + 1] * L[S_B + 1] + L[S_B + 2] * L[S_B + 2]);
       eintr = eintr - 0.5 * (R[S_B] * R[S_B] + R[S_B + 1] * R[S_B + 1] + R[S_B + 2] * R[S_B + 2]);
     }
-    const double em = pm[Q_EINT * QS], e0 = p0[Q_EINT * QS], ep = pp[Q_EINT * QS];
+    const double em = pm[Lay<MAG>::EINT * QS], e0 = p0[Lay<MAG>::EINT * QS], ep = pp[Lay<MAG>::EINT * QS];
     if (eintl >= fmax2(em, e0) || eintl <= fmin2(em, e0) || eintr >= fmax2(e0, ep) || eintr <= fmin2(e0, ep)) {
 #pragma unroll
       for (int q = 0; q < NS; q++) sl[q] = 0.0;
@@ -68,7 +68,7 @@ __device__ __forceinline__ void slopes_with(const double* pm, const double* p0, 
   }
 }
 
-// The slopes with IEEE division, out of line: the rare path of slopes_of.
+// The slopes with IEEE division, out of line: the rare path of slopes_fast.
 // Slope q goes to out[q * os].
 template <bool MAG, int LIM, int QS>
 __device__ __noinline__ void slopes_ieee(const double* pm, const double* p0, const double* pp, const AxisGeo* g,
@@ -77,7 +77,7 @@ __device__ __noinline__ void slopes_ieee(const double* pm, const double* p0, con
   double sl[NS];
   slopes_with<MAG, LIM, QS>(pm, p0, pp, *g, cg, sl, pd);
 #pragma unroll
-  for (int q = 0; q < NS; q++) out[q * os] = sl[q];
+  for (int q = 0; q < Lay<MAG>::NS; q++) out[q * os] = sl[q];
 }
 
 // The slopes with every quotient formed by FastDiv, recomputed with IEEE
@@ -97,29 +97,15 @@ __device__ __noinline__ void slopes_fast(const double* pm, const double* p0, con
     return;
   }
 #pragma unroll
-  for (int q = 0; q < NS; q++) out[q * os] = sl[q];
+  for (int q = 0; q < Lay<MAG>::NS; q++) out[q * os] = sl[q];
 }
-template <bool MAG, int LIM, int QS>
-__device__ __forceinline__ void slopes_of(const double* pm, const double* p0, const double* pp, const AxisGeo& g,
-                                          int cg, double sl[NS]) {
-  if constexpr (LIM == 0) {
-#pragma unroll
-    for (int q = 0; q < NS; q++) sl[q] = 0.0;
-  } else {
-    double tmp[NS];
-    slopes_fast<MAG, LIM, QS>(pm, p0, pp, &g, cg, tmp, 1);
-#pragma unroll
-    for (int q = 0; q < NS; q++) sl[q] = tmp[q];
-  }
-}
-
-// slopes_of written straight to out[q * os] (shared memory).
+// The slopes written straight to out[q * os] (shared memory).
 template <bool MAG, int LIM, int QS>
 __device__ __forceinline__ void slopes_to(const double* pm, const double* p0, const double* pp, const AxisGeo& g,
                                           int cg, double* out, int os) {
   if constexpr (LIM == 0) {
 #pragma unroll
-    for (int q = 0; q < NS; q++) out[q * os] = 0.0;
+    for (int q = 0; q < Lay<MAG>::NS; q++) out[q * os] = 0.0;
   } else {
     slopes_fast<MAG, LIM, QS>(pm, p0, pp, &g, cg, out, os);
   }
@@ -189,28 +175,25 @@ __device__ __forceinline__ bool face_flux_with(PL pl, PR pr, SL sl, SR sr, doubl
   return true;
 }
 
-// Store a face flux: with os == 0, fl in the solver's order to out[0..8];
-// otherwise rotated back into the conserved slots (numflux.f90:186-198,
-// 359-371, 531-543), slot v to out[v * os].
+// Store a face flux rotated back into the conserved slots
+// (numflux.f90:186-198, 359-371, 531-543), slot v to out[v * os].
+template <bool MAG>
 __device__ __forceinline__ void put_flux(const double fl[9], int cn, int c1, int c2, double* out, int os) {
-  if (os == 0) {
-#pragma unroll
-    for (int q = 0; q < 9; q++) out[q] = fl[q];
-    return;
-  }
   out[ICNT * os] = fl[0];
   out[(IMO1 + cn) * os] = fl[1];
   out[(IMO1 + c1) * os] = fl[2];
   out[(IMO1 + c2) * os] = fl[3];
   out[IENE * os] = fl[4];
-  out[(IMG1 + cn) * os] = fl[5];
-  out[(IMG1 + c1) * os] = fl[6];
-  out[(IMG1 + c2) * os] = fl[7];
-  out[I9WV * os] = fl[8];
+  if constexpr (MAG) {
+    out[(IMG1 + cn) * os] = fl[5];
+    out[(IMG1 + c1) * os] = fl[6];
+    out[(IMG1 + c2) * os] = fl[7];
+    out[I9WV * os] = fl[8];
+  }
 }
 
 // The face flux with IEEE division, out of line: the rare path of
-// face_flux.  pl/pr: staged quantity 0 of the cells (stride QS); sl/sr:
+// face_flux_fast.  pl/pr: staged quantity 0 of the cells (stride QS); sl/sr:
 // slope 0 (strides ssl, ssr); out/os as put_flux.
 template <bool MAG, int QS>
 __device__ __noinline__ bool face_flux_ieee(const double* pl, const double* pr, const double* sl, int ssl,
@@ -221,7 +204,7 @@ __device__ __noinline__ bool face_flux_ieee(const double* pl, const double* pr, 
   const bool ok = face_flux_with<MAG>([&](int q) { return pl[q * QS]; }, [&](int q) { return pr[q * QS]; },
                                       [&](int q) { return sl[q * ssl]; }, [&](int q) { return sr[q * ssr]; }, dx1,
                                       dx2, cn, c1, c2, gamma, gm1, ch, fl, pd);
-  put_flux(fl, cn, c1, c2, out, os);
+  put_flux<MAG>(fl, cn, c1, c2, out, os);
   return ok;
 }
 
@@ -241,7 +224,7 @@ __device__ __noinline__ bool face_flux_fast(const double* pl, const double* pr, 
                                       dx2, cn, c1, c2, gamma, gm1, ch, fl, fd);
   if (fd.bad)
     return face_flux_ieee<MAG, QS>(pl, pr, sl, ssl, sr, ssr, dx1, dx2, cn, c1, c2, gamma, gm1, ch, out, os);
-  put_flux(fl, cn, c1, c2, out, os);
+  put_flux<MAG>(fl, cn, c1, c2, out, os);
   return ok;
 }
 

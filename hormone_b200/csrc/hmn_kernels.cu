@@ -39,20 +39,25 @@
 
 namespace hmn {
 
+// G and A stay in the parameter bank: the out-of-line slope and face calls
+// take the address of an axis's description, and without __grid_constant__
+// that makes every thread copy all of G to its stack first
 template <bool MAG, bool GLM, class TL, bool SPH = false, bool PUSH = false>
-__global__ void __launch_bounds__(TL::NT, TL::MINB) stage_kernel(const GridDev G, const StageArgs A) {
+__global__ void __launch_bounds__(TL::NT, (MAG ? TL::MINB : TL::MINBH)) stage_kernel(const __grid_constant__ GridDev G,
+                                                                           const __grid_constant__ StageArgs A) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  SmemT<TL>& sm = *reinterpret_cast<SmemT<TL>*>(smem_raw);
+  SmemT<TL, MAG>& sm = *reinterpret_cast<SmemT<TL, MAG>*>(smem_raw);
   if (A.sc->done) return;
   stage_tile_exact<MAG, GLM, TL, SPH, PUSH>(G, A, sm, blockIdx.x, nullptr);
 }
 
 // the same stage with the stencil region staged by TMA (3-D tiles)
 template <bool MAG, bool GLM, class TL>
-__global__ void __launch_bounds__(TL::NT, TL::MINB)
-    stage_kernel_tma(const GridDev G, const StageArgs A, const __grid_constant__ TmaMaps tm) {
+__global__ void __launch_bounds__(TL::NT, (MAG ? TL::MINB : TL::MINBH))
+    stage_kernel_tma(const __grid_constant__ GridDev G, const __grid_constant__ StageArgs A,
+                     const __grid_constant__ TmaMaps tm) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  SmemT<TL>& sm = *reinterpret_cast<SmemT<TL>*>(smem_raw);
+  SmemT<TL, MAG>& sm = *reinterpret_cast<SmemT<TL, MAG>*>(smem_raw);
   if (A.sc->done) return;
   // bulk tensor copies need 128-byte aligned destinations (uniform over the CTA)
   const bool tma = (smem_addr(&sm.P[0][0]) & 127u) == 0;
@@ -145,7 +150,7 @@ __global__ void advance_kernel(DevScalars* sc) {
 // spherical grids: the plain (non-TMA) FP64 kernel with the metric factors
 template <bool MAG, bool GLM, class TL>
 static cudaError_t launch_stage_sph(const GridDev& G, const StageArgs& A, cudaStream_t st) {
-  constexpr int smem = (int)sizeof(SmemT<TL>);
+  constexpr int smem = (int)sizeof(SmemT<TL, MAG>);
   const int blocks = A.tiles[0] * A.tiles[1] * A.tiles[2];
   static bool attr = false;
   if (!attr) {
@@ -158,7 +163,11 @@ static cudaError_t launch_stage_sph(const GridDev& G, const StageArgs& A, cudaSt
   return cudaGetLastError();
 }
 
-// r always solved; 1-D grids carry no GLM wave, 2-D and 3-D MHD grids do
+// r always solved; 1-D grids carry no GLM wave, 2-D and 3-D MHD grids do.
+// Without a field the smaller layout lets one CTA more share an SM, at fewer
+// registers; with the grid description read from the parameter bank instead
+// of a stack copy per thread, the 128x64x128 star takes 13.3 ms for 8 steps
+// instead of 18.0.
 template <class TL>
 static cudaError_t launch_stage_sph_tl(const GridDev& G, const StageArgs& A, bool mag, bool glm, cudaStream_t st) {
   constexpr bool multi = (TL::TY > 1) || (TL::TZ > 1);
@@ -171,16 +180,16 @@ static cudaError_t launch_stage_spherical(const GridDev& G, const StageArgs& A, 
   const int* t = A.tile;
   if (A.nspc > 0) return cudaErrorInvalidValue;
   if (t[0] == 8 && t[1] == 8 && t[2] == 8) return launch_stage_sph_tl<Tile<8, 8, 8, 640, 1>>(G, A, mag, glm, st);
-  if (t[0] == 8 && t[1] == 8 && t[2] == 4) return launch_stage_sph_tl<Tile<8, 8, 4, 384, 2>>(G, A, mag, glm, st);
-  if (t[0] == 16 && t[1] == 16 && t[2] == 1) return launch_stage_sph_tl<Tile<16, 16, 1, 288, 2>>(G, A, mag, glm, st);
-  if (t[0] == 16 && t[1] == 1 && t[2] == 16) return launch_stage_sph_tl<Tile<16, 1, 16, 288, 2>>(G, A, mag, glm, st);
-  if (t[0] == 256 && t[1] == 1 && t[2] == 1) return launch_stage_sph_tl<Tile<256, 1, 1, 288, 2>>(G, A, mag, glm, st);
+  if (t[0] == 8 && t[1] == 8 && t[2] == 4) return launch_stage_sph_tl<Tile<8, 8, 4, 384, 2, 0, 3>>(G, A, mag, glm, st);
+  if (t[0] == 16 && t[1] == 16 && t[2] == 1) return launch_stage_sph_tl<Tile<16, 16, 1, 288, 2, 0, 3>>(G, A, mag, glm, st);
+  if (t[0] == 16 && t[1] == 1 && t[2] == 16) return launch_stage_sph_tl<Tile<16, 1, 16, 288, 2, 0, 3>>(G, A, mag, glm, st);
+  if (t[0] == 256 && t[1] == 1 && t[2] == 1) return launch_stage_sph_tl<Tile<256, 1, 1, 288, 2, 0, 3>>(G, A, mag, glm, st);
   return cudaErrorInvalidValue;
 }
 
 template <bool MAG, bool GLM, class TL>
 static cudaError_t launch_stage_t(const GridDev& G, const StageArgs& A, const TmaMaps* tm, cudaStream_t st) {
-  constexpr int smem = (int)sizeof(SmemT<TL>);
+  constexpr int smem = (int)sizeof(SmemT<TL, MAG>);
   const int blocks = A.tiles[0] * A.tiles[1] * A.tiles[2];
   if constexpr (TL::HX && TL::HY && TL::HZ) {  // TMA staging needs halos on all three axes
     if (tm != nullptr) {
@@ -245,7 +254,7 @@ void stage_tile(const int solve[3], int precision, int nspc, int tile[3], bool s
 // boundary layers into the neighbours' halo buffers (3-D Cartesian tiles)
 template <bool MAG, bool GLM, class TL>
 static cudaError_t launch_stage_push_t(const GridDev& G, const StageArgs& A, cudaStream_t st) {
-  constexpr int smem = (int)sizeof(SmemT<TL>);
+  constexpr int smem = (int)sizeof(SmemT<TL, MAG>);
   const int blocks = A.tiles[0] * A.tiles[1] * A.tiles[2];
   static bool attr = false;
   if (!attr) {
@@ -276,18 +285,20 @@ static cudaError_t launch_stage_push(const GridDev& G, const StageArgs& A, bool 
 }
 
 // The stage tiles whose shared-memory layout has room for SP passive
-// scalars (8 x 8 x 4 in 3-D; with 8 scalars its 203 KB allow one CTA per SM)
+// scalars (8 x 8 x 4 in 3-D; with 8 scalars its 203 KB allow one CTA per SM;
+// one CTA more in 2-D without a field: 501x350 cells with two scalars, 32
+// steps 10.8 -> 7.1 ms together with the parameter bank reads)
 template <int SP, int MINB3>
 static cudaError_t launch_scalar_tiles(const GridDev& G, const StageArgs& A, bool mag, bool glm, cudaStream_t st) {
   const int* t = A.tile;
   if (t[0] == 8 && t[1] == 8 && t[2] == 4)
     return launch_stage_tl<Tile<8, 8, 4, 384, MINB3, SP>>(G, A, mag, glm, nullptr, st);
   if (t[0] == 16 && t[1] == 16 && t[2] == 1)
-    return launch_stage_tl<Tile<16, 16, 1, 288, MINB3, SP>>(G, A, mag, glm, nullptr, st);
+    return launch_stage_tl<Tile<16, 16, 1, 288, MINB3, SP, MINB3 + 1>>(G, A, mag, glm, nullptr, st);
   if (t[0] == 16 && t[1] == 1 && t[2] == 16)
-    return launch_stage_tl<Tile<16, 1, 16, 288, MINB3, SP>>(G, A, mag, glm, nullptr, st);
+    return launch_stage_tl<Tile<16, 1, 16, 288, MINB3, SP, MINB3 + 1>>(G, A, mag, glm, nullptr, st);
   if (t[0] == 1 && t[1] == 16 && t[2] == 16)
-    return launch_stage_tl<Tile<1, 16, 16, 288, MINB3, SP>>(G, A, mag, glm, nullptr, st);
+    return launch_stage_tl<Tile<1, 16, 16, 288, MINB3, SP, MINB3 + 1>>(G, A, mag, glm, nullptr, st);
   if (t[0] == 256 && t[1] == 1 && t[2] == 1) return launch_stage_tl<Tile<256, 1, 1, 288, 2, SP>>(G, A, mag, glm, nullptr, st);
   if (t[0] == 1 && t[1] == 256 && t[2] == 1) return launch_stage_tl<Tile<1, 256, 1, 288, 2, SP>>(G, A, mag, glm, nullptr, st);
   if (t[0] == 1 && t[1] == 1 && t[2] == 256) return launch_stage_tl<Tile<1, 1, 256, 288, 2, SP>>(G, A, mag, glm, nullptr, st);
@@ -309,12 +320,12 @@ cudaError_t launch_stage(const GridDev& G, const StageArgs& A, bool mag, bool gl
   }
   if (t[0] == 8 && t[1] == 8 && t[2] == 8) return launch_stage_tl<Tile<8, 8, 8, 640, 1>>(G, A, mag, glm, tm, st);
   if (t[0] == 8 && t[1] == 8 && t[2] == 4) return launch_stage_tl<Tile<8, 8, 4, 384, 2>>(G, A, mag, glm, tm, st);
-  if (t[0] == 16 && t[1] == 16 && t[2] == 1) return launch_stage_tl<Tile<16, 16, 1, 288, 3>>(G, A, mag, glm, nullptr, st);
-  if (t[0] == 16 && t[1] == 1 && t[2] == 16) return launch_stage_tl<Tile<16, 1, 16, 288, 3>>(G, A, mag, glm, nullptr, st);
-  if (t[0] == 1 && t[1] == 16 && t[2] == 16) return launch_stage_tl<Tile<1, 16, 16, 288, 3>>(G, A, mag, glm, nullptr, st);
-  if (t[0] == 256 && t[1] == 1 && t[2] == 1) return launch_stage_tl<Tile<256, 1, 1, 288, 3>>(G, A, mag, glm, nullptr, st);
-  if (t[0] == 1 && t[1] == 256 && t[2] == 1) return launch_stage_tl<Tile<1, 256, 1, 288, 3>>(G, A, mag, glm, nullptr, st);
-  if (t[0] == 1 && t[1] == 1 && t[2] == 256) return launch_stage_tl<Tile<1, 1, 256, 288, 3>>(G, A, mag, glm, nullptr, st);
+  if (t[0] == 16 && t[1] == 16 && t[2] == 1) return launch_stage_tl<Tile<16, 16, 1, 288, 3, 0, 4>>(G, A, mag, glm, nullptr, st);
+  if (t[0] == 16 && t[1] == 1 && t[2] == 16) return launch_stage_tl<Tile<16, 1, 16, 288, 3, 0, 4>>(G, A, mag, glm, nullptr, st);
+  if (t[0] == 1 && t[1] == 16 && t[2] == 16) return launch_stage_tl<Tile<1, 16, 16, 288, 3, 0, 4>>(G, A, mag, glm, nullptr, st);
+  if (t[0] == 256 && t[1] == 1 && t[2] == 1) return launch_stage_tl<Tile<256, 1, 1, 288, 3, 0, 4>>(G, A, mag, glm, nullptr, st);
+  if (t[0] == 1 && t[1] == 256 && t[2] == 1) return launch_stage_tl<Tile<1, 256, 1, 288, 3, 0, 4>>(G, A, mag, glm, nullptr, st);
+  if (t[0] == 1 && t[1] == 1 && t[2] == 256) return launch_stage_tl<Tile<1, 1, 256, 288, 3, 0, 4>>(G, A, mag, glm, nullptr, st);
   return cudaErrorInvalidValue;
 }
 
@@ -475,10 +486,10 @@ cudaError_t launch_advance(DevScalars* sc, cudaStream_t st) {
 // in its descriptor, so a batch step equals one hormone.f90 step per grid.
 
 using T3D = Tile<8, 8, 8, 640, 1>;
-using T3D4 = Tile<8, 8, 4, 384, 2>;
-using T2D = Tile<16, 16, 1, 288, 3>;
-using T2D8 = Tile<32, 8, 1, 320, 3>;
-using T1D = Tile<256, 1, 1, 288, 3>;
+using T3D4 = Tile<8, 8, 4, 384, 2, 0, 3>;
+using T2D = Tile<16, 16, 1, 288, 3, 0, 4>;
+using T2D8 = Tile<32, 8, 1, 320, 3, 0, 4>;
+using T1D = Tile<256, 1, 1, 288, 3, 0, 4>;
 
 // tile ids: 0 3-D 8x8x8 (640 threads), 1 3-D 8x8x4 (256 threads, 2 CTAs/SM),
 // 2 2-D 16x16, 3 2-D 32x8, 4 1-D 256.  batch_tile_kind gives the grid's
@@ -513,10 +524,10 @@ void batch_tile_shape(int tid, int tile[3]) {
 }
 
 template <bool MAG, bool GLM, class TL, bool DYN>
-__global__ void __launch_bounds__(TL::NT, TL::MINB) batch_stage_kernel(SimDesc* sims, const int2* items, int nitems,
+__global__ void __launch_bounds__(TL::NT, (MAG ? TL::MINB : TL::MINBH)) batch_stage_kernel(SimDesc* sims, const int2* items, int nitems,
                                                                         int stage, int rk, int* queue) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  SmemT<TL>& sm = *reinterpret_cast<SmemT<TL>*>(smem_raw);
+  SmemT<TL, MAG>& sm = *reinterpret_cast<SmemT<TL, MAG>*>(smem_raw);
   for_each_item<DYN>(nitems, queue, [&](int it) {
     const int2 w = items[it];
     SimDesc& S = sims[w.x];
@@ -590,10 +601,10 @@ static cudaError_t batch_attr_t() {
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(batch_stage_kernel<MAG, GLM, TL, false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemT<TL>));
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemT<TL, MAG>));
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(batch_stage_kernel<MAG, GLM, TL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sizeof(SmemT<TL>));
+                               (int)sizeof(SmemT<TL, MAG>));
     if (e != cudaSuccess) return e;
     attr = true;
   }
@@ -607,10 +618,10 @@ static cudaError_t launch_batch_stage_t(SimDesc* sims, const int2* items, int ni
   if (e != cudaSuccess) return e;
   if (queue)
     batch_stage_kernel<MAG, GLM, TL, true>
-        <<<grid, TL::NT, sizeof(SmemT<TL>), st>>>(sims, items, nitems, stage, rk, queue);
+        <<<grid, TL::NT, sizeof(SmemT<TL, MAG>), st>>>(sims, items, nitems, stage, rk, queue);
   else
     batch_stage_kernel<MAG, GLM, TL, false>
-        <<<grid, TL::NT, sizeof(SmemT<TL>), st>>>(sims, items, nitems, stage, rk, nullptr);
+        <<<grid, TL::NT, sizeof(SmemT<TL, MAG>), st>>>(sims, items, nitems, stage, rk, nullptr);
   return cudaGetLastError();
 }
 
@@ -641,7 +652,7 @@ static int occupancy_t() {
   int n = 0;
   batch_attr_t<MAG, GLM, TL>();
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_stage_kernel<MAG, GLM, TL, true>, TL::NT,
-                                                sizeof(SmemT<TL>));  // the static split's shared memory is no larger
+                                                sizeof(SmemT<TL, MAG>));  // the static split's shared memory is no larger
   return n > 0 ? n : 1;
 }
 

@@ -53,11 +53,13 @@ namespace hmn {
 namespace {
 
 // TX x TY columns (one owner thread each), NH more threads, MINB resident
-// CTAs per SM.  OXY: the owners also take x-y slope and face items (the last
-// NC of each list), for tiles whose other threads are fewer than the items.
-template <int TX_, int TY_, int NH_, int MINB_, bool OXY_>
+// CTAs per SM (MINBH on grids without a field).  OXY: the owners also take
+// x-y slope and face items (the last NC of each list), for tiles whose other
+// threads are fewer than the items.
+template <int TX_, int TY_, int NH_, int MINB_, bool OXY_, int MINBH_ = MINB_>
 struct March {
-  static constexpr int TX = TX_, TY = TY_, NC = TX * TY, NH = NH_, NT = NC + NH, MINB = MINB_;
+  static constexpr int TX = TX_, TY = TY_, NC = TX * TY, NH = NH_, NT = NC + NH;
+  static constexpr int MINB = MINB_, MINBH = MINBH_;  // with a field; without one
   static constexpr bool OXY = OXY_;
   // staged cells of one plane: rows j in [0, TY) extended by two cells in x,
   // then the two rows below the tile and the two above (no corners)
@@ -82,13 +84,13 @@ struct March {
   }
 };
 
-template <class MT>
+template <class MT, bool MAG>
 struct MarchSmem {
-  double W[3][NQ][MT::NPL];    // rolling window: plane p in slot (p - k0 + 2) % 3
-  double S[NS][MT::NSXY];      // x slopes ((TX+2) x TY), then y slopes (TX x (TY+2)) of plane k
-  double F[9][MT::NFXY];       // x faces ((TX+1) x TY), then y faces (TX x (TY+1)) of plane k
-  double SZ[NS][MT::NC];       // per column: the z slope of plane k
-  double FZ[9][MT::NC];        // per column: the z flux through face k-1/2
+  double W[3][Lay<MAG>::NQ][MT::NPL];  // rolling window: plane p in slot (p - k0 + 2) % 3
+  double S[Lay<MAG>::NS][MT::NSXY];    // x slopes ((TX+2) x TY), then y slopes (TX x (TY+2)) of plane k
+  double F[Lay<MAG>::NF][MT::NFXY];    // x faces ((TX+1) x TY), then y faces (TX x (TY+1)) of plane k
+  double SZ[Lay<MAG>::NS][MT::NC];     // per column: the z slope of plane k
+  double FZ[Lay<MAG>::NF][MT::NC];     // per column: the z flux through face k-1/2
 };
 
 // Stage plane p into window slot W (cells first, first + stride, ...): every
@@ -112,7 +114,8 @@ __device__ __forceinline__ void stage_plane(const GridDev& G, const StageArgs& A
     double q[NQ];
     stage_cell<MAG, GLM>(G, A, x0 + i, y0 + j, p, q);
 #pragma unroll
-    for (int s = 0; s < NQ; s++) W[s][w] = q[s];
+    for (int s = 0; s < NQ; s++)
+      if (Lay<MAG>::slot(s) >= 0) W[Lay<MAG>::slot(s)][w] = q[s];
   }
 }
 
@@ -165,7 +168,7 @@ __device__ __forceinline__ void cart_gravity(const GridDev& G, const StageArgs& 
 // lands in fz already rotated into the conserved slots (put_flux with unit
 // stride; numflux.f90:531-543).
 template <bool MAG, class MT>
-__device__ __forceinline__ bool z_face(const double* Wk, const double* Wk1, const MarchSmem<MT>& sm, int t,
+__device__ __forceinline__ bool z_face(const double* Wk, const double* Wk1, const MarchSmem<MT, MAG>& sm, int t,
                                        const double* sr, const AxisGeo& gz, int k, const StageArgs& A, double ch,
                                        double fz[9]) {
   constexpr int QS = MT::NPL;
@@ -177,11 +180,11 @@ __device__ __forceinline__ bool z_face(const double* Wk, const double* Wk1, cons
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.L2 [%0];" ::"l"(p)); }
 
 template <bool MAG, bool GLM, int LIM, class MT, bool PUSH>
-__global__ void __launch_bounds__(MT::NT, MT::MINB)
+__global__ void __launch_bounds__(MT::NT, (MAG ? MT::MINB : MT::MINBH))
     march_stage_kernel(const __grid_constant__ GridDev G, const __grid_constant__ StageArgs A, int LZ, int ntx,
                        int nty) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  MarchSmem<MT>& sm = *reinterpret_cast<MarchSmem<MT>*>(smem_raw);
+  MarchSmem<MT, MAG>& sm = *reinterpret_cast<MarchSmem<MT, MAG>*>(smem_raw);
   if (A.sc->done) return;
   constexpr int TX = MT::TX, TY = MT::TY, NC = MT::NC, NH = MT::NH, NT = MT::NT, QS = MT::NPL;
   constexpr int nv = MAG ? (GLM ? 9 : 8) : 5;
@@ -217,7 +220,7 @@ __global__ void __launch_bounds__(MT::NT, MT::MINB)
   __syncthreads();
   if (live) {
 #pragma unroll
-    for (int q = 0; q < NS; q++) sm.SZ[q][tid] = szn[q];  // the slope of k0-1 is the face's left slope
+    for (int q = 0; q < Lay<MAG>::NS; q++) sm.SZ[q][tid] = szn[q];  // the slope of k0-1 is the face's left slope
     double szk[NS];
     slopes_to<MAG, LIM, QS>(&sm.W[slot(k0 - 1)][0][orr], &sm.W[slot(k0)][0][orr], &sm.W[slot(k0 + 1)][0][orr], gz,
                             k0, szk, 1);
@@ -226,12 +229,12 @@ __global__ void __launch_bounds__(MT::NT, MT::MINB)
       record_error(A.sc, kENEG_EINT, x0 + oi, y0 + oj, k0 - 1);
     if (k0 == 0 && G.fb != nullptr) {  // boundary code 10 at the inner z face (fluxboundary.f90:42-87)
 #pragma unroll
-      for (int q = 0; q < 9; q++) fz[q] = G.fb[q];
+      for (int q = 0; q < Lay<MAG>::NF; q++) fz[q] = G.fb[q];
     }
 #pragma unroll
-    for (int q = 0; q < NS; q++) sm.SZ[q][tid] = szk[q];
+    for (int q = 0; q < Lay<MAG>::NS; q++) sm.SZ[q][tid] = szk[q];
 #pragma unroll
-    for (int q = 0; q < 9; q++) sm.FZ[q][tid] = fz[q];
+    for (int q = 0; q < Lay<MAG>::NF; q++) sm.FZ[q][tid] = fz[q];
   }
   __syncthreads();
   stage_plane<MAG, GLM, MT>(G, A, sm.W[slot(k0 + 2)], k0 + 2, k0 + 2 < kend, x0, y0, T0, T1, tid, NT);
@@ -302,12 +305,12 @@ __global__ void __launch_bounds__(MT::NT, MT::MINB)
         record_error(A.sc, kENEG_EINT, x0 + oi, y0 + oj, k);
       const double idz = gz.idxi[k + 2];
 #pragma unroll
-      for (int q = 0; q < 9; q++) {
+      for (int q = 0; q < Lay<MAG>::NF; q++) {
         dz[q] = idz * (sm.FZ[q][tid] - fz[q]);
         sm.FZ[q][tid] = fz[q];
       }
 #pragma unroll
-      for (int q = 0; q < NS; q++) sm.SZ[q][tid] = szn[q];
+      for (int q = 0; q < Lay<MAG>::NS; q++) sm.SZ[q][tid] = szn[q];
     }
     // owners, then: one x-y face each (the last NC of the list); the other
     // threads: the rest of the list
@@ -418,12 +421,15 @@ __global__ void __launch_bounds__(MT::NT, MT::MINB)
 }
 
 // 16x8 columns with 128 more threads; the owners take x-y items too, so
-// every thread has one to two items per phase
-using MT168 = March<16, 8, 128, 2, true>;
+// every thread has one to two items per phase.  Without a field the phases
+// are short and wait on latency and barriers, and the layout takes 66 KB
+// instead of 111: three CTAs per SM at 80 registers (the 160^3 polytrope, 8
+// steps with copies: 56.1 -> 51.1 ms).
+using MT168 = March<16, 8, 128, 2, true, 3>;
 
 template <bool MAG, bool GLM, int LIM, bool PUSH, class MT>
 cudaError_t launch_mt(const GridDev& G, const StageArgs& A, int LZ, int ntx, int nty, int nch, cudaStream_t st) {
-  constexpr int smem = (int)sizeof(MarchSmem<MT>);
+  constexpr int smem = (int)sizeof(MarchSmem<MT, MAG>);
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(march_stage_kernel<MAG, GLM, LIM, MT, PUSH>,

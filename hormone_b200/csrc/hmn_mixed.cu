@@ -31,11 +31,11 @@
 
 namespace hmn {
 
-template <class TL>
+template <class TL, bool MAG>
 struct SmemMixed {
-  double P[NQ][TL::NR];  // first: every TMA box destination in it is 128-byte aligned
-  float S[NS][TL::NSB];
-  float F[9][TL::NFB];
+  double P[Lay<MAG>::NQ][TL::NR];  // first: every TMA box destination in it is 128-byte aligned
+  float S[Lay<MAG>::NS][TL::NSB];
+  float F[Lay<MAG>::NF][TL::NFB];
   uint64_t bar;          // completion barrier of the region's bulk copies
 };
 
@@ -70,7 +70,7 @@ __device__ __forceinline__ double minmod_fast(double u0, double u1, double u2, d
 }
 
 template <int AX, bool MAG, bool GLM, class TL, bool SPH = false>
-__device__ __forceinline__ void axis_pass_mixed(const GridDev& G, const StageArgs& A, SmemMixed<TL>& sm,
+__device__ __forceinline__ void axis_pass_mixed(const GridDev& G, const StageArgs& A, SmemMixed<TL, MAG>& sm,
                                                 const int t0[3], const int T[3], double acc[9], float ch) {
   constexpr int TX = TL::TX, TY = TL::TY, TZ = TL::TZ;
   constexpr int SBX = TX + (AX == 0 ? 2 : 0), SBY = TY + (AX == 1 ? 2 : 0), SBZ = TZ + (AX == 2 ? 2 : 0);
@@ -131,7 +131,7 @@ __device__ __forceinline__ void axis_pass_mixed(const GridDev& G, const StageArg
         eintl = eintl - 0.5 * (L[S_B] * L[S_B] + L[S_B + 1] * L[S_B + 1] + L[S_B + 2] * L[S_B + 2]);
         eintr = eintr - 0.5 * (R[S_B] * R[S_B] + R[S_B + 1] * R[S_B + 1] + R[S_B + 2] * R[S_B + 2]);
       }
-      const double em = sm.P[Q_EINT][rm], e0 = sm.P[Q_EINT][r], ep = sm.P[Q_EINT][rp];
+      const double em = sm.P[Lay<MAG>::EINT][rm], e0 = sm.P[Lay<MAG>::EINT][r], ep = sm.P[Lay<MAG>::EINT][rp];
       if (eintl >= fmax2(em, e0) || eintl <= fmin2(em, e0) || eintr >= fmax2(e0, ep) || eintr <= fmin2(e0, ep)) {
 #pragma unroll
         for (int q = 0; q < NS; q++) sl[q] = 0.0;
@@ -216,7 +216,7 @@ __device__ __forceinline__ void axis_pass_mixed(const GridDev& G, const StageArg
     }
     if (AX == 2 && G.fb != nullptr && t0[2] + f == 0) {  // boundary code 10 (fluxboundary.f90:42-87)
 #pragma unroll
-      for (int q = 0; q < 9; q++) sm.F[q][w] = (float)G.fb[q];
+      for (int q = 0; q < Lay<MAG>::NF; q++) sm.F[q][w] = (float)G.fb[q];
       continue;
     }
     sm.F[ICNT][w] = fl[0];
@@ -262,7 +262,7 @@ __device__ __forceinline__ void axis_pass_mixed(const GridDev& G, const StageArg
 // One tile of one RK stage; `tile_id` enumerates the tiles of the grid
 // (x fastest).  Shared by the single-grid and the batched kernels.
 template <bool MAG, bool GLM, class TL, bool SPH = false, bool PUSH = false>
-__device__ __forceinline__ void stage_tile_mixed(const GridDev& G, const StageArgs& A, SmemMixed<TL>& sm, int tile_id,
+__device__ __forceinline__ void stage_tile_mixed(const GridDev& G, const StageArgs& A, SmemMixed<TL, MAG>& sm, int tile_id,
                                                  const TmaMaps* tm) {
   const int tid = threadIdx.x;
   int bid = tile_id;
@@ -389,19 +389,19 @@ __device__ __forceinline__ void stage_tile_mixed(const GridDev& G, const StageAr
 }
 
 template <bool MAG, bool GLM, class TL, bool SPH = false, bool PUSH = false>
-__global__ void __launch_bounds__(TL::NT, TL::MINB) stage_kernel_mixed(const GridDev G, const StageArgs A) {
+__global__ void __launch_bounds__(TL::NT, (MAG ? TL::MINB : TL::MINBH)) stage_kernel_mixed(const GridDev G, const StageArgs A) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  SmemMixed<TL>& sm = *reinterpret_cast<SmemMixed<TL>*>(smem_raw);
+  SmemMixed<TL, MAG>& sm = *reinterpret_cast<SmemMixed<TL, MAG>*>(smem_raw);
   if (A.sc->done) return;
   stage_tile_mixed<MAG, GLM, TL, SPH, PUSH>(G, A, sm, blockIdx.x, nullptr);
 }
 
 // the same stage with the stencil region staged by TMA (3-D tiles)
 template <bool MAG, bool GLM, class TL>
-__global__ void __launch_bounds__(TL::NT, TL::MINB)
+__global__ void __launch_bounds__(TL::NT, (MAG ? TL::MINB : TL::MINBH))
     stage_kernel_mixed_tma(const GridDev G, const StageArgs A, const __grid_constant__ TmaMaps tm) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  SmemMixed<TL>& sm = *reinterpret_cast<SmemMixed<TL>*>(smem_raw);
+  SmemMixed<TL, MAG>& sm = *reinterpret_cast<SmemMixed<TL, MAG>*>(smem_raw);
   if (A.sc->done) return;
   const bool tma = (smem_addr(&sm.P[0][0]) & 127u) == 0;
   stage_tile_mixed<MAG, GLM, TL>(G, A, sm, blockIdx.x, tma ? &tm : nullptr);
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(TL::NT, TL::MINB)
 
 template <bool MAG, bool GLM, class TL>
 static cudaError_t launch_mixed_t(const GridDev& G, const StageArgs& A, const TmaMaps* tm, cudaStream_t st) {
-  constexpr int smem = (int)sizeof(SmemMixed<TL>);
+  constexpr int smem = (int)sizeof(SmemMixed<TL, MAG>);
   const int blocks = A.tiles[0] * A.tiles[1] * A.tiles[2];
   if constexpr (TL::HX && TL::HY && TL::HZ) {  // TMA staging needs halos on all three axes
     if (tm != nullptr) {
@@ -446,7 +446,7 @@ static cudaError_t launch_mixed_tl(const GridDev& G, const StageArgs& A, bool ma
 // spherical grids: the plain (non-TMA) mixed kernel with the metric factors
 template <bool MAG, bool GLM, class TL>
 static cudaError_t launch_mixed_sph(const GridDev& G, const StageArgs& A, cudaStream_t st) {
-  constexpr int smem = (int)sizeof(SmemMixed<TL>);
+  constexpr int smem = (int)sizeof(SmemMixed<TL, MAG>);
   const int blocks = A.tiles[0] * A.tiles[1] * A.tiles[2];
   static bool attr = false;
   if (!attr) {
@@ -481,7 +481,7 @@ static cudaError_t launch_mixed_spherical(const GridDev& G, const StageArgs& A, 
 // z slabs exchanging by push (see push_boundary_layers): 3-D Cartesian tiles
 template <bool MAG, bool GLM, class TL>
 static cudaError_t launch_mixed_push_t(const GridDev& G, const StageArgs& A, cudaStream_t st) {
-  constexpr int smem = (int)sizeof(SmemMixed<TL>);
+  constexpr int smem = (int)sizeof(SmemMixed<TL, MAG>);
   const int blocks = A.tiles[0] * A.tiles[1] * A.tiles[2];
   static bool attr = false;
   if (!attr) {
@@ -524,11 +524,11 @@ cudaError_t launch_stage_mixed(const GridDev& G, const StageArgs& A, bool mag, b
 
 // batched form (see batch_stage_kernel in hmn_kernels.cu)
 template <bool MAG, bool GLM, class TL, bool DYN>
-__global__ void __launch_bounds__(TL::NT, TL::MINB) batch_stage_kernel_mixed(SimDesc* sims, const int2* items,
+__global__ void __launch_bounds__(TL::NT, (MAG ? TL::MINB : TL::MINBH)) batch_stage_kernel_mixed(SimDesc* sims, const int2* items,
                                                                               int nitems, int stage, int rk,
                                                                               int* queue) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  SmemMixed<TL>& sm = *reinterpret_cast<SmemMixed<TL>*>(smem_raw);
+  SmemMixed<TL, MAG>& sm = *reinterpret_cast<SmemMixed<TL, MAG>*>(smem_raw);
   for_each_item<DYN>(nitems, queue, [&](int it) {
     const int2 w = items[it];
     SimDesc& S = sims[w.x];
@@ -550,10 +550,10 @@ static cudaError_t bm_attr_t() {
   static bool attr = false;
   if (!attr) {
     cudaError_t e = cudaFuncSetAttribute(batch_stage_kernel_mixed<MAG, GLM, TL, false>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemMixed<TL>));
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemMixed<TL, MAG>));
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(batch_stage_kernel_mixed<MAG, GLM, TL, true>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemMixed<TL>));
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemMixed<TL, MAG>));
     if (e != cudaSuccess) return e;
     attr = true;
   }
@@ -567,10 +567,10 @@ static cudaError_t launch_bm_t(SimDesc* sims, const int2* items, int nitems, int
   if (e != cudaSuccess) return e;
   if (queue)
     batch_stage_kernel_mixed<MAG, GLM, TL, true>
-        <<<grid, TL::NT, sizeof(SmemMixed<TL>), st>>>(sims, items, nitems, stage, rk, queue);
+        <<<grid, TL::NT, sizeof(SmemMixed<TL, MAG>), st>>>(sims, items, nitems, stage, rk, queue);
   else
     batch_stage_kernel_mixed<MAG, GLM, TL, false>
-        <<<grid, TL::NT, sizeof(SmemMixed<TL>), st>>>(sims, items, nitems, stage, rk, nullptr);
+        <<<grid, TL::NT, sizeof(SmemMixed<TL, MAG>), st>>>(sims, items, nitems, stage, rk, nullptr);
   return cudaGetLastError();
 }
 
@@ -599,7 +599,7 @@ static int occ_m() {
   int n = 0;
   bm_attr_t<MAG, GLM, TL>();
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_stage_kernel_mixed<MAG, GLM, TL, true>, TL::NT,
-                                                sizeof(SmemMixed<TL>));  // the static split's is no larger
+                                                sizeof(SmemMixed<TL, MAG>));  // the static split's is no larger
   return n > 0 ? n : 1;
 }
 

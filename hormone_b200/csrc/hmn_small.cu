@@ -73,7 +73,7 @@ template <bool MAG, bool GLM, class TL, bool SPH>
 __global__ void __launch_bounds__(TL::NT, 1)
     small_run_kernel(const __grid_constant__ GridDev G, const __grid_constant__ SmallRun R) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  SmemT<TL>& sm = *reinterpret_cast<SmemT<TL>*>(smem_raw);
+  SmemT<TL, MAG>& sm = *reinterpret_cast<SmemT<TL, MAG>*>(smem_raw);
   DevScalars* sc = R.sc;
   if (*(volatile int*)&sc->done) return;
   unsigned int nb = 0;  // barriers passed (the same count in every CTA)
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(TL::NT, 1)
 
 template <bool MAG, bool GLM, class TL, bool SPH>
 cudaError_t launch_t(const GridDev& G, const SmallRun& R, cudaStream_t st, int* grid_out) {
-  constexpr int smem = (int)sizeof(SmemT<TL>);
+  constexpr int smem = (int)sizeof(SmemT<TL, MAG>);
   auto fn = small_run_kernel<MAG, GLM, TL, SPH>;
   static int per_sm = -1;
   if (per_sm < 0) {

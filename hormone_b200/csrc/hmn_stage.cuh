@@ -15,18 +15,18 @@
 
 namespace hmn {
 
-template <class TL>
+template <class TL, bool MAG>
 struct SmemT {
-  double P[NQ + TL::SP][TL::NR];  // first: every TMA box destination in it is 128-byte aligned
-  double S[NS + TL::SP][TL::NSB];
-  double F[9 + TL::SP][TL::NFB];
+  double P[Lay<MAG>::NQ + TL::SP][TL::NR];  // first: every TMA box destination in it is 128-byte aligned
+  double S[Lay<MAG>::NS + TL::SP][TL::NSB];
+  double F[Lay<MAG>::NF + TL::SP][TL::NFB];
   uint64_t bar;                   // completion barrier of the region's bulk copies
 };
 
 // One axis of the fused stage: slopes, face fluxes, flux divergence of the
 // thread's own cell added to acc[].
 template <int AX, bool MAG, bool GLM, class TL, bool SPH = false>
-__device__ __forceinline__ void axis_pass(const GridDev& G, const StageArgs& A, SmemT<TL>& sm, const int t0[3],
+__device__ __forceinline__ void axis_pass(const GridDev& G, const StageArgs& A, SmemT<TL, MAG>& sm, const int t0[3],
                                           const int T[3], double acc[9], double accs[], double ch) {
   constexpr int TX = TL::TX, TY = TL::TY, TZ = TL::TZ;
   constexpr int SBX = TX + (AX == 0 ? 2 : 0), SBY = TY + (AX == 1 ? 2 : 0), SBZ = TZ + (AX == 2 ? 2 : 0);
@@ -64,13 +64,13 @@ __device__ __forceinline__ void axis_pass(const GridDev& G, const StageArgs& A, 
       for (int n = 0; n < A.nspc; n++) {
         double du = 0.0;
         if (A.limiter != 0) {
-          const double u0 = sm.P[NQ + n][rm], u1 = sm.P[NQ + n][r], u2 = sm.P[NQ + n][rp];
+          const double u0 = sm.P[Lay<MAG>::NQ + n][rm], u1 = sm.P[Lay<MAG>::NQ + n][r], u2 = sm.P[Lay<MAG>::NQ + n][rp];
           if (A.limiter == 1)
             du = lim_minmod(u0, u1, u2, g.idx[cg + 2], g.idx[cg + 3], g.isum[cg + 2]);
           else
             du = lim_mmc(u0, u1, u2, g.mcf[cg + 2], g.mcb[cg + 2], g.ga[cg + 2], g.gb[cg + 2]);
         }
-        sm.S[NS + n][w] = du;
+        sm.S[Lay<MAG>::NS + n][w] = du;
       }
     }
   }
@@ -104,9 +104,9 @@ __device__ __forceinline__ void axis_pass(const GridDev& G, const StageArgs& A, 
     // (numflux.f90:566 -> fluxboundary.f90:42-87)
     if (AX == 2 && G.fb != nullptr && t0[2] + f == 0) {
 #pragma unroll
-      for (int q = 0; q < 9; q++) sm.F[q][w] = G.fb[q];
+      for (int q = 0; q < Lay<MAG>::NF; q++) sm.F[q][w] = G.fb[q];
       if constexpr (TL::SP > 0)
-        for (int n = 0; n < A.nspc; n++) sm.F[9 + n][w] = G.fb[9 + n];
+        for (int n = 0; n < A.nspc; n++) sm.F[Lay<MAG>::NF + n][w] = G.fb[9 + n];
       continue;
     }
     // passive scalars: face fractions upwinded by the mass flux and
@@ -118,8 +118,8 @@ __device__ __forceinline__ void axis_pass(const GridDev& G, const StageArgs& A, 
 #pragma unroll
         for (int n = 0; n < TL::SP; n++) {
           if (n < A.nspc) {
-            spl[n] = sm.P[NQ + n][rL] + dx1 * sm.S[NS + n][sL];
-            spr[n] = sm.P[NQ + n][rR] - dx2 * sm.S[NS + n][sR];
+            spl[n] = sm.P[Lay<MAG>::NQ + n][rL] + dx1 * sm.S[Lay<MAG>::NS + n][sL];
+            spr[n] = sm.P[Lay<MAG>::NQ + n][rR] - dx2 * sm.S[Lay<MAG>::NS + n][sR];
             suml = suml + spl[n];
             sumr = sumr + spr[n];
           }
@@ -129,7 +129,7 @@ __device__ __forceinline__ void axis_pass(const GridDev& G, const StageArgs& A, 
         const double fix = 1.0 / (suml * (0.5 + sg) + sumr * (0.5 - sg));
 #pragma unroll
         for (int n = 0; n < TL::SP; n++)
-          if (n < A.nspc) sm.F[9 + n][w] = fix * f0 * (spl[n] * (0.5 + sg) + spr[n] * (0.5 - sg));
+          if (n < A.nspc) sm.F[Lay<MAG>::NF + n][w] = fix * f0 * (spl[n] * (0.5 + sg) + spr[n] * (0.5 - sg));
       }
     }
   }
@@ -157,7 +157,7 @@ __device__ __forceinline__ void axis_pass(const GridDev& G, const StageArgs& A, 
         const double idxi = g.idxi[cc[AX] + t0[AX] + 2];
 #pragma unroll
         for (int n = 0; n < TL::SP; n++)
-          if (n < A.nspc) accs[n] = accs[n] + idxi * (sm.F[9 + n][wm] - sm.F[9 + n][wp]);
+          if (n < A.nspc) accs[n] = accs[n] + idxi * (sm.F[Lay<MAG>::NF + n][wm] - sm.F[Lay<MAG>::NF + n][wp]);
       }
     }
   }
@@ -178,7 +178,7 @@ __device__ __forceinline__ bool cfl_values(const GridDev& G, double gamma, doubl
 // CFLOUT: also fold dti and the signal speed of each new cell (dti_cell,
 // the next step's CFL reduction) into *cdti (min) and *ccf (max).
 template <bool MAG, bool GLM, class TL, bool SPH = false, bool PUSH = false, bool CFLOUT = false>
-__device__ __forceinline__ void stage_tile_exact(const GridDev& G, const StageArgs& A, SmemT<TL>& sm, int tile_id,
+__device__ __forceinline__ void stage_tile_exact(const GridDev& G, const StageArgs& A, SmemT<TL, MAG>& sm, int tile_id,
                                                  const TmaMaps* tm, double* cdti = nullptr, double* ccf = nullptr) {
   const int tid = threadIdx.x;
 

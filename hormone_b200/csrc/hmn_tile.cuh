@@ -20,6 +20,19 @@ enum { Q_D = 0, Q_M = 1, Q_E = 4, Q_B = 5, Q_PHI = 8, Q_EINT = 9, NQ = 10 };
 // slopes: d, e, m1..3, b1..3
 enum { S_D = 0, S_E = 1, S_M = 2, S_B = 5, NS = 8 };
 
+// What a tile keeps per cell, slope cell and face in shared memory: without a
+// field only the hydrodynamic part of the lists above (6, 5 and 5 instead of
+// 10, 8 and 9), which leaves room for more CTAs per SM.
+template <bool MAG>
+struct Lay {
+  static constexpr int NQ = MAG ? hmn::NQ : 6;       // staged quantities
+  static constexpr int EINT = MAG ? Q_EINT : 5;      // slot of eint among them
+  static constexpr int NS = MAG ? hmn::NS : S_B;     // slopes
+  static constexpr int NF = MAG ? 9 : 5;             // conserved slots of a face flux
+  // slot of quantity q, or -1 where it is not kept
+  __host__ __device__ static constexpr int slot(int q) { return MAG || q < Q_B ? q : (q == Q_EINT ? EINT : -1); }
+};
+
 
 __device__ __forceinline__ void record_error(DevScalars* sc, int code, int i, int j, int k) {
   if (atomicCAS(&sc->err_code, 0, code) == 0) {
@@ -35,7 +48,7 @@ __device__ __forceinline__ size_t cidx(const GridDev& G, int i, int j, int k) {
 
 // Compile-time description of a tile: TX x TY x TZ cells (256 in all) and a
 // halo of two cells beyond each face of every axis with extent > 1.
-template <int TX_, int TY_, int TZ_, int NT_ = 256, int MINB_ = 2, int SP_ = 0>
+template <int TX_, int TY_, int TZ_, int NT_ = 256, int MINB_ = 2, int SP_ = 0, int MINBH_ = MINB_>
 struct Tile {
   static constexpr int TX = TX_, TY = TY_, TZ = TZ_;
   static constexpr int SP = SP_;      // passive scalars the shared-memory layout has room for
@@ -43,7 +56,8 @@ struct Tile {
   // largest per-axis slope box, so that every phase of an axis pass takes one
   // round (16x16 -> 288, 256 -> 288, 32x8 -> 320, 8x8x4 -> 384, 8x8x8 -> 640)
   static constexpr int NT = NT_;
-  static constexpr int MINB = MINB_;  // resident CTAs per SM the register budget is sized for
+  // resident CTAs per SM the register budget is sized for, with and without a field
+  static constexpr int MINB = MINB_, MINBH = MINBH_;
   static constexpr int NC = TX * TY * TZ;
   static constexpr int HX = TX > 1 ? 2 : 0, HY = TY > 1 ? 2 : 0, HZ = TZ > 1 ? 2 : 0;
   // region part 0: x-extended rows of every interior (j,k); part 1: y halos; part 2: z halos
@@ -329,12 +343,14 @@ __device__ __forceinline__ void stage_region(const GridDev& G, const StageArgs& 
     }
     __syncthreads();
     if (tid == 0) {
-      mbar_arrive_expect_tx(bar, (uint32_t)(NQ * TL::NR * sizeof(double)));
+      mbar_arrive_expect_tx(bar, (uint32_t)(Lay<MAG>::NQ * TL::NR * sizeof(double)));
       // HBM plane p -> staged slot (d, v1..3 (made m below), e, b1..3, phi, eint)
       constexpr int dst[NP] = {Q_D, Q_M, Q_M + 1, Q_M + 2, Q_E, Q_B, Q_B + 1, Q_B + 2, Q_PHI, Q_EINT};
 #pragma unroll
       for (int p = 0; p < NP; p++) {
-        double* base = P[dst[p]];
+        const int sl = Lay<MAG>::slot(dst[p]);
+        if (sl < 0) continue;
+        double* base = P[sl];
         tma_load_4d(base, &tm->box[0], bar, t0[0] - 2, t0[1], t0[2], p);
         tma_load_4d(base + TL::N0, &tm->box[1], bar, t0[0], t0[1] - 2, t0[2], p);
         tma_load_4d(base + TL::N0 + TL::N1 / 2, &tm->box[1], bar, t0[0], t0[1] + TL::TY, t0[2], p);
@@ -372,27 +388,27 @@ __device__ __forceinline__ void stage_region(const GridDev& G, const StageArgs& 
       P[Q_M + 0][w] = d * P[Q_M + 0][w];
       P[Q_M + 1][w] = d * P[Q_M + 1][w];
       P[Q_M + 2][w] = d * P[Q_M + 2][w];
-      if (!MAG) P[Q_B + 0][w] = P[Q_B + 1][w] = P[Q_B + 2][w] = 0.0;
-      P[Q_PHI][w] = GLM ? P[Q_PHI][w] * A.phifac : 0.0;
+      if constexpr (MAG) P[Q_PHI][w] = GLM ? P[Q_PHI][w] * A.phifac : 0.0;
       continue;
     }
     double q[NQ];
     stage_cell<MAG, GLM>(G, A, gi, gj, gk, q);
 #pragma unroll
-    for (int s = 0; s < NQ; s++) P[s][w] = q[s];
+    for (int s = 0; s < NQ; s++)
+      if (Lay<MAG>::slot(s) >= 0) P[Lay<MAG>::slot(s)][w] = q[s];
     if constexpr (TL::SP > 0) {
       const int zio = gk < 0 ? 0 : 1;
       if ((gk < 0 || gk >= G.n[2]) && G.zhalo[zio] != nullptr) {  // neighbouring slab
         const size_t hp = (size_t)G.n[0] * G.n[1];
         const size_t h = (size_t)(zio == 0 ? gk + 2 : gk - G.n[2]) * hp + (size_t)gi + (size_t)G.n[0] * gj;
-        for (int n = 0; n < A.nspc; n++) P[NQ + n][w] = G.zhalo[zio][(size_t)(NP + n) * 2 * hp + h];
+        for (int n = 0; n < A.nspc; n++) P[Lay<MAG>::NQ + n][w] = G.zhalo[zio][(size_t)(NP + n) * 2 * hp + h];
       } else if (const double* D = dirichlet_face(G, gi, gj, gk)) {
         const size_t hd = dirichlet_index(G, gi, gj, gk);
         const size_t two_area = 2 * dirichlet_area(G, gi, gj, gk);
-        for (int n = 0; n < A.nspc; n++) P[NQ + n][w] = D[(size_t)(8 + n) * two_area + hd];
+        for (int n = 0; n < A.nspc; n++) P[Lay<MAG>::NQ + n][w] = D[(size_t)(8 + n) * two_area + hd];
       } else {
         const size_t cs = scalar_image(G, gi, gj, gk);
-        for (int n = 0; n < A.nspc; n++) P[NQ + n][w] = A.pin[(size_t)(NP + n) * A.plane + cs];
+        for (int n = 0; n < A.nspc; n++) P[Lay<MAG>::NQ + n][w] = A.pin[(size_t)(NP + n) * A.plane + cs];
       }
     }
   }
