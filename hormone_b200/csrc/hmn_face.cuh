@@ -13,13 +13,27 @@
 namespace hmn {
 namespace {
 
+// What every face of a launch (of a simulation, in a batch) shares: a copy in
+// shared memory, so that the face function takes one pointer instead of four
+// values in registers.
+struct FluxConst {
+  double gamma, gm1, ch, rch;  // rch: 1/ch, correctly rounded
+};
+__device__ __forceinline__ void set_flux_const(FluxConst& fc, const StageArgs& A) {
+  const double ch = A.sc->ch;
+  fc.gamma = A.gamma;
+  fc.gm1 = A.gm1;
+  fc.ch = ch;
+  fc.rch = 1.0 / ch;
+}
+
 // Limited slopes of one cell along one axis from its two neighbours
 // (interpolation.f90:49-163 with fluxlimiter.f90:40-75): pm, p0, pp point at
-// staged quantity 0 of the cells, quantity q at [q * QS].  cg is the cell's
-// global coordinate along the axis.  The same operations as axis_pass.
+// staged quantity 0 of the cells, quantity q at [q * QS].  g points at the
+// cell in the axis's first array, array q at g[q * len] (GEO_*).
 template <bool MAG, int LIM, int QS, class D>
-__device__ __forceinline__ void slopes_with(const double* pm, const double* p0, const double* pp, const AxisGeo& g,
-                                            int cg, double sl[NS], D& dv) {
+__device__ __forceinline__ void slopes_with(const double* pm, const double* p0, const double* pp, const double* g,
+                                            int len, double sl[NS], D& dv) {
   constexpr int nsl = MAG ? NS : S_B;
 #pragma unroll
   for (int q = 0; q < NS; q++) sl[q] = 0.0;
@@ -27,10 +41,10 @@ __device__ __forceinline__ void slopes_with(const double* pm, const double* p0, 
     return;
   } else {
     constexpr int qmap[NS] = {Q_D, Q_E, Q_M + 0, Q_M + 1, Q_M + 2, Q_B + 0, Q_B + 1, Q_B + 2};
-    const double hl = g.hl[cg + 2], hr = g.hr[cg + 2];
+    const double hl = g[GEO_HL * len], hr = g[GEO_HR * len];
     double L[NS], R[NS];
     if constexpr (LIM == 1) {
-      const double i0 = g.idx[cg + 2], i1 = g.idx[cg + 3], is = g.isum[cg + 2];
+      const double i0 = g[GEO_IDX * len], i1 = g[GEO_IDX * len + 1], is = g[GEO_ISUM * len];
       const double ris = dv.rec(is);
 #pragma unroll
       for (int q = 0; q < nsl; q++) {
@@ -41,7 +55,7 @@ __device__ __forceinline__ void slopes_with(const double* pm, const double* p0, 
         R[q] = u1 + hr * du;
       }
     } else {
-      const double cf = g.mcf[cg + 2], cb = g.mcb[cg + 2], ga = g.ga[cg + 2], gb = g.gb[cg + 2];
+      const double cf = g[GEO_MCF * len], cb = g[GEO_MCB * len], ga = g[GEO_GA * len], gb = g[GEO_GB * len];
       const double rga = dv.rec(ga), rgb = dv.rec(gb);
 #pragma unroll
       for (int q = 0; q < nsl; q++) {
@@ -68,46 +82,57 @@ __device__ __forceinline__ void slopes_with(const double* pm, const double* p0, 
   }
 }
 
+// What a caller of the out-of-line functions below vouches for: staged cells,
+// slopes and fluxes lie in shared memory.  (A pointer argument is generic; with
+// this the accesses need no address-space test.)
+__device__ __forceinline__ void in_shared(const void* p) { __builtin_assume(__isShared(p)); }
+
 // The slopes with IEEE division, out of line: the rare path of slopes_fast.
-// Slope q goes to out[q * os].
-template <bool MAG, int LIM, int QS>
-__device__ __noinline__ void slopes_ieee(const double* pm, const double* p0, const double* pp, const AxisGeo* g,
-                                         int cg, double* out, int os) {
+// Slope q goes to out[q * OS].
+template <bool MAG, int LIM, int QS, int OS>
+__device__ __noinline__ void slopes_ieee(const double* pm, const double* p0, const double* pp, const double* g, int L,
+                                         double* out) {
   PlainDiv pd;
   double sl[NS];
-  slopes_with<MAG, LIM, QS>(pm, p0, pp, *g, cg, sl, pd);
+  slopes_with<MAG, LIM, QS>(pm, p0, pp, g, L, sl, pd);
 #pragma unroll
-  for (int q = 0; q < Lay<MAG>::NS; q++) out[q * os] = sl[q];
+  for (int q = 0; q < Lay<MAG>::NS; q++) out[q * OS] = sl[q];
 }
 
 // The slopes with every quotient formed by FastDiv, recomputed with IEEE
 // division where FastDiv could not vouch for one (bitwise the same result).
-// One out-of-line copy serves every call site, so that warps in different
-// phases of the march share instruction cache lines.  Slope q goes to
-// out[q * os]: a caller that keeps slopes in shared memory passes its slot
-// there, and nothing goes through the stack.
-template <bool MAG, int LIM, int QS>
-__device__ __noinline__ void slopes_fast(const double* pm, const double* p0, const double* pp, const AxisGeo* g,
-                                         int cg, double* out, int os) {
+// One out-of-line copy serves every call site of a kernel, so that warps in
+// different phases share instruction cache lines.  Slope q goes straight to
+// out[q * OS]: with every stride a constant and the axis's arrays reached from
+// one pointer, a call spends no multiplications on addresses and loads no
+// pointer that it then has to wait for.  (Before, with run-time strides, four
+// solver constants in registers and the march's z slopes and fluxes on the
+// stack: 256^3 MHD stage 7.10 -> 6.60 ms, 97x75x62 box 15.2 -> 14.3 ms for 16
+// steps, 160^3 polytrope 51.1 -> 48.5 ms.)
+template <bool MAG, int LIM, int QS, int OS>
+__device__ __noinline__ void slopes_fast(const double* pm, const double* p0, const double* pp, const double* g, int L,
+                                         double* out) {
+  in_shared(pm), in_shared(p0), in_shared(pp), in_shared(out);
   FastDiv fd;
   double sl[NS];
-  slopes_with<MAG, LIM, QS>(pm, p0, pp, *g, cg, sl, fd);
+  slopes_with<MAG, LIM, QS>(pm, p0, pp, g, L, sl, fd);
   if (fd.bad) {
-    slopes_ieee<MAG, LIM, QS>(pm, p0, pp, g, cg, out, os);
+    slopes_ieee<MAG, LIM, QS, OS>(pm, p0, pp, g, L, out);
     return;
   }
 #pragma unroll
-  for (int q = 0; q < Lay<MAG>::NS; q++) out[q * os] = sl[q];
+  for (int q = 0; q < Lay<MAG>::NS; q++) out[q * OS] = sl[q];
 }
-// The slopes written straight to out[q * os] (shared memory).
-template <bool MAG, int LIM, int QS>
-__device__ __forceinline__ void slopes_to(const double* pm, const double* p0, const double* pp, const AxisGeo& g,
-                                          int cg, double* out, int os) {
+
+// The slopes of the cell at global coordinate cg along the axis, n cells long.
+template <bool MAG, int LIM, int QS, int OS>
+__device__ __forceinline__ void slopes_to(const double* pm, const double* p0, const double* pp, const AxisGeo& g, int n,
+                                          int cg, double* out) {
   if constexpr (LIM == 0) {
 #pragma unroll
-    for (int q = 0; q < Lay<MAG>::NS; q++) out[q * os] = 0.0;
+    for (int q = 0; q < Lay<MAG>::NS; q++) out[q * OS] = 0.0;
   } else {
-    slopes_fast<MAG, LIM, QS>(pm, p0, pp, &g, cg, out, os);
+    slopes_fast<MAG, LIM, QS, OS>(pm, p0, pp, g.x + cg + 2, n + 4, out);
   }
 }
 
@@ -120,7 +145,8 @@ __device__ __forceinline__ void slopes_to(const double* pm, const double* p0, co
 // rho <= 0 (numflux.f90:117 -> error_flux).
 template <bool MAG, class D, class PL, class PR, class SL, class SR>
 __device__ __forceinline__ bool face_flux_with(PL pl, PR pr, SL sl, SR sr, double dx1, double dx2, int cn, int c1,
-                                               int c2, double gamma, double gm1, double ch, double fl[9], D& dv) {
+                                               int c2, const FluxConst& fc, double fl[9], D& dv) {
+  const double gamma = fc.gamma, gm1 = fc.gm1;
   const double dl = pl(Q_D) + dx1 * sl(S_D);
   const double dr = pr(Q_D) - dx2 * sr(S_D);
   const double el = pl(Q_E) + dx1 * sl(S_E);
@@ -170,61 +196,71 @@ __device__ __forceinline__ bool face_flux_with(PL pl, PR pr, SL sl, SR sr, doubl
   const double ptr = ptr0 + 0.5 * (b1r * b1r + b2r * b2r + b3r * b3r);
   const double cfl = get_cf(dl, csl, b1l, b2l, b3l, dv, rdl);
   const double cfr = get_cf(dr, csr, b1r, b2r, b3r, dv, rdr);
+  const double ch = fc.ch;
+  dv.template need_pos<-500, 501>(ch);
   hlld(fl, cfl, cfr, v1l, v1r, v2l, v2r, v3l, v3r, dl, dr, el, er, ptl, ptr, b1l, b1r, b2l, b2r, b3l, b3r, phil, phir,
-       ch, dv);
+       ch, fc.rch, dv);
   return true;
 }
 
 // Store a face flux rotated back into the conserved slots
-// (numflux.f90:186-198, 359-371, 531-543), slot v to out[v * os].
-template <bool MAG>
-__device__ __forceinline__ void put_flux(const double fl[9], int cn, int c1, int c2, double* out, int os) {
-  out[ICNT * os] = fl[0];
-  out[(IMO1 + cn) * os] = fl[1];
-  out[(IMO1 + c1) * os] = fl[2];
-  out[(IMO1 + c2) * os] = fl[3];
-  out[IENE * os] = fl[4];
+// (numflux.f90:186-198, 359-371, 531-543), slot v to out[v * OS].
+template <bool MAG, int OS>
+__device__ __forceinline__ void put_flux(const double fl[9], int cn, int c1, int c2, double* out) {
+  double *on = out + cn * OS, *o1 = out + c1 * OS, *o2 = out + c2 * OS;
+  out[ICNT * OS] = fl[0];
+  on[IMO1 * OS] = fl[1];
+  o1[IMO1 * OS] = fl[2];
+  o2[IMO1 * OS] = fl[3];
+  out[IENE * OS] = fl[4];
   if constexpr (MAG) {
-    out[(IMG1 + cn) * os] = fl[5];
-    out[(IMG1 + c1) * os] = fl[6];
-    out[(IMG1 + c2) * os] = fl[7];
-    out[I9WV * os] = fl[8];
+    on[IMG1 * OS] = fl[5];
+    o1[IMG1 * OS] = fl[6];
+    o2[IMG1 * OS] = fl[7];
+    out[I9WV * OS] = fl[8];
   }
 }
 
+// The flux through a face normal to axis cn from staged cells (quantity 0 at
+// pl, pr, stride QS) and slopes (slope 0 at sl, sr, stride SS).
+template <bool MAG, int QS, int SS, class D>
+__device__ __forceinline__ bool face_flux_at(const double* pl, const double* pr, const double* sl, const double* sr,
+                                             double dx1, double dx2, int cn, int c1, int c2, const FluxConst* fc,
+                                             double fl[9], D& dv) {
+  return face_flux_with<MAG>([&](int q) { return pl[q * QS]; }, [&](int q) { return pr[q * QS]; },
+                             [&](int q) { return sl[q * SS]; }, [&](int q) { return sr[q * SS]; }, dx1, dx2, cn, c1,
+                             c2, *fc, fl, dv);
+}
+
 // The face flux with IEEE division, out of line: the rare path of
-// face_flux_fast.  pl/pr: staged quantity 0 of the cells (stride QS); sl/sr:
-// slope 0 (strides ssl, ssr); out/os as put_flux.
-template <bool MAG, int QS>
-__device__ __noinline__ bool face_flux_ieee(const double* pl, const double* pr, const double* sl, int ssl,
-                                            const double* sr, int ssr, double dx1, double dx2, int cn, int c1, int c2,
-                                            double gamma, double gm1, double ch, double* out, int os) {
+// face_flux_fast; arguments as there.
+template <bool MAG, int QS, int SS, int OS>
+__device__ __noinline__ bool face_flux_ieee(const double* pl, const double* pr, const double* sl, const double* sr,
+                                            double dx1, double dx2, int cn, const FluxConst* fc, double* out) {
   PlainDiv pd;
+  const int c1 = cn == 2 ? 0 : cn + 1, c2 = cn == 0 ? 2 : cn - 1;
   double fl[9];
-  const bool ok = face_flux_with<MAG>([&](int q) { return pl[q * QS]; }, [&](int q) { return pr[q * QS]; },
-                                      [&](int q) { return sl[q * ssl]; }, [&](int q) { return sr[q * ssr]; }, dx1,
-                                      dx2, cn, c1, c2, gamma, gm1, ch, fl, pd);
-  put_flux<MAG>(fl, cn, c1, c2, out, os);
+  const bool ok = face_flux_at<MAG, QS, SS>(pl, pr, sl, sr, dx1, dx2, cn, c1, c2, fc, fl, pd);
+  put_flux<MAG, OS>(fl, cn, c1, c2, out);
   return ok;
 }
 
 // The face flux with every quotient formed by FastDiv, recomputed with IEEE
 // division where FastDiv could not vouch for one (bitwise the same result);
-// one out-of-line copy for the x, y and z faces.  Arguments as
-// face_flux_ieee.  A caller that keeps fluxes in shared memory passes its
-// slot and stride, and nothing goes through the stack.
-template <bool MAG, int QS>
-__device__ __noinline__ bool face_flux_fast(const double* pl, const double* pr, const double* sl, int ssl,
-                                            const double* sr, int ssr, double dx1, double dx2, int cn, int c1, int c2,
-                                            double gamma, double gm1, double ch, double* out, int os) {
+// one out-of-line copy for the x, y and z faces of a kernel.  The flux goes to
+// out[slot * OS]; out may be where sl or sr is, for every operand is read
+// before the first store.  Returns false (flux zero) where a face state has
+// eint <= 0 or rho <= 0.
+template <bool MAG, int QS, int SS, int OS>
+__device__ __noinline__ bool face_flux_fast(const double* pl, const double* pr, const double* sl, const double* sr,
+                                            double dx1, double dx2, int cn, const FluxConst* fc, double* out) {
+  in_shared(pl), in_shared(pr), in_shared(sl), in_shared(sr), in_shared(fc), in_shared(out);
   FastDiv fd;
+  const int c1 = cn == 2 ? 0 : cn + 1, c2 = cn == 0 ? 2 : cn - 1;
   double fl[9];
-  const bool ok = face_flux_with<MAG>([&](int q) { return pl[q * QS]; }, [&](int q) { return pr[q * QS]; },
-                                      [&](int q) { return sl[q * ssl]; }, [&](int q) { return sr[q * ssr]; }, dx1,
-                                      dx2, cn, c1, c2, gamma, gm1, ch, fl, fd);
-  if (fd.bad)
-    return face_flux_ieee<MAG, QS>(pl, pr, sl, ssl, sr, ssr, dx1, dx2, cn, c1, c2, gamma, gm1, ch, out, os);
-  put_flux<MAG>(fl, cn, c1, c2, out, os);
+  const bool ok = face_flux_at<MAG, QS, SS>(pl, pr, sl, sr, dx1, dx2, cn, c1, c2, fc, fl, fd);
+  if (fd.bad) return face_flux_ieee<MAG, QS, SS, OS>(pl, pr, sl, sr, dx1, dx2, cn, fc, out);
+  put_flux<MAG, OS>(fl, cn, c1, c2, out);
   return ok;
 }
 

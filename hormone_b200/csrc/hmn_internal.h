@@ -13,6 +13,10 @@ namespace hmn {
 // the caller passes, with the same single IEEE operations the reference
 // performs inside its loops, so that reading them is bit-equivalent to
 // recomputing them.
+// Position of an axis's arrays in its block of kGeoArrays x (n + 4) doubles
+// (AxisGeo's pointers, in order): array q of cell s is x[q * (n + 4) + s + 2].
+enum { GEO_HL = 5, GEO_HR = 6, GEO_IDX = 2, GEO_MCF = 7, GEO_MCB = 8, GEO_GA = 9, GEO_GB = 10, GEO_ISUM = 11 };
+
 struct AxisGeo {
   const double* x;     // cell centres
   const double* dx;    // centre spacing dx(c) = x(c)-x(c-1) as the grid defines it

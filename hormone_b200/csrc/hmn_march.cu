@@ -26,10 +26,9 @@
 // shared memory (108 KB: three 16x8 planes with their x-y halo, x-y slopes
 // and fluxes of one plane, the z slopes and fluxes of one plane) lets two
 // CTAs share an SM, so one CTA's barrier waits overlap the other's work.
-// The z quantities of a column never leave the thread that owns it: its z
-// slope crosses one barrier in registers and then waits in shared memory for
-// the next plane, its z flux waits in shared memory, and the z flux
-// difference is applied by the same thread in phase 3.
+// The z quantities of a column stay with the thread that owns it: its z
+// slopes and z flux wait in shared memory slots that only this thread uses,
+// and it applies the z flux difference in phase 3.
 //
 // Quotients: the stage is bound by the issue of dependent FP64 instructions,
 // and about 190 of them per cell are IEEE divisions, most sharing a
@@ -53,14 +52,12 @@ namespace hmn {
 namespace {
 
 // TX x TY columns (one owner thread each), NH more threads, MINB resident
-// CTAs per SM (MINBH on grids without a field).  OXY: the owners also take
-// x-y slope and face items (the last NC of each list), for tiles whose other
-// threads are fewer than the items.
-template <int TX_, int TY_, int NH_, int MINB_, bool OXY_, int MINBH_ = MINB_>
+// CTAs per SM (MINBH on grids without a field).  The owners also take x-y
+// slope and face items, the last NC of each list.
+template <int TX_, int TY_, int NH_, int MINB_, int MINBH_>
 struct March {
   static constexpr int TX = TX_, TY = TY_, NC = TX * TY, NH = NH_, NT = NC + NH;
   static constexpr int MINB = MINB_, MINBH = MINBH_;  // with a field; without one
-  static constexpr bool OXY = OXY_;
   // staged cells of one plane: rows j in [0, TY) extended by two cells in x,
   // then the two rows below the tile and the two above (no corners)
   static constexpr int NROW = (TX + 4) * TY;
@@ -84,13 +81,22 @@ struct March {
   }
 };
 
+// Slopes and fluxes share one row length, so that every stride of the slope
+// and face functions is the same constant.  A column's z slope of plane k+1
+// passes phase 1 to phase 2 in the flux slots of its owner's x-y face (ZT),
+// which that thread fills only after its z face; the z flux comes back in the
+// slots of the z slope it used up.  Nothing of the z sweep passes through the
+// stack.
 template <class MT, bool MAG>
 struct MarchSmem {
+  static constexpr int XY = 0, FXY = MT::NSXY, SZ = FXY + MT::NFXY, FZ = SZ + MT::NC, ROW = FZ + MT::NC;
+  static constexpr int ZT = FXY + MT::NFXY - MT::NC;
   double W[3][Lay<MAG>::NQ][MT::NPL];  // rolling window: plane p in slot (p - k0 + 2) % 3
-  double S[Lay<MAG>::NS][MT::NSXY];    // x slopes ((TX+2) x TY), then y slopes (TX x (TY+2)) of plane k
-  double F[Lay<MAG>::NF][MT::NFXY];    // x faces ((TX+1) x TY), then y faces (TX x (TY+1)) of plane k
-  double SZ[Lay<MAG>::NS][MT::NC];     // per column: the z slope of plane k
-  double FZ[Lay<MAG>::NF][MT::NC];     // per column: the z flux through face k-1/2
+  // per row q: the slope q of the x and then the y slope cells of plane k, the
+  // flux slot q of its x and then its y faces, and per column the z slope of
+  // plane k and the z flux through face k-1/2
+  double R[Lay<MAG>::NF][ROW];
+  FluxConst fc;
 };
 
 // Stage plane p into window slot W (cells first, first + stride, ...): every
@@ -162,18 +168,14 @@ __device__ __forceinline__ void cart_gravity(const GridDev& G, const StageArgs& 
 }
 
 // z flux of the face above the column's cell (k+1/2) from the window: the
-// left state from plane k with the z slope the column keeps in SZ, the
-// right one from plane k+1 with its slope in the thread's array sr (which
-// the slope call filled in place: it is handed on, not copied).  The flux
-// lands in fz already rotated into the conserved slots (put_flux with unit
-// stride; numflux.f90:531-543).
+// left state from plane k with the z slope at sl, the right one from plane
+// k+1 with the slope at sr.  The flux lands in out already rotated into the
+// conserved slots (numflux.f90:531-543).
 template <bool MAG, class MT>
-__device__ __forceinline__ bool z_face(const double* Wk, const double* Wk1, const MarchSmem<MT, MAG>& sm, int t,
-                                       const double* sr, const AxisGeo& gz, int k, const StageArgs& A, double ch,
-                                       double fz[9]) {
-  constexpr int QS = MT::NPL;
-  const double dx1 = gz.hr[k + 2], dx2 = gz.hl[k + 3];
-  return face_flux_fast<MAG, QS>(Wk, Wk1, &sm.SZ[0][t], MT::NC, sr, 1, dx1, dx2, 2, 0, 1, A.gamma, A.gm1, ch, fz, 1);
+__device__ __forceinline__ bool z_face(const double* Wk, const double* Wk1, const double* sl, const double* sr,
+                                       const AxisGeo& gz, int k, const FluxConst* fc, double* out) {
+  constexpr int RS = MarchSmem<MT, MAG>::ROW;
+  return face_flux_fast<MAG, MT::NPL, RS, RS>(Wk, Wk1, sl, sr, gz.hr[k + 2], gz.hl[k + 3], 2, fc, out);
 }
 
 // Ask for the line of p to be brought into L2 (no register, no wait).
@@ -184,9 +186,11 @@ __global__ void __launch_bounds__(MT::NT, (MAG ? MT::MINB : MT::MINBH))
     march_stage_kernel(const __grid_constant__ GridDev G, const __grid_constant__ StageArgs A, int LZ, int ntx,
                        int nty) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  MarchSmem<MT, MAG>& sm = *reinterpret_cast<MarchSmem<MT, MAG>*>(smem_raw);
+  using SM = MarchSmem<MT, MAG>;
+  SM& sm = *reinterpret_cast<SM*>(smem_raw);
   if (A.sc->done) return;
-  constexpr int TX = MT::TX, TY = MT::TY, NC = MT::NC, NH = MT::NH, NT = MT::NT, QS = MT::NPL;
+  constexpr int TX = MT::TX, TY = MT::TY, NC = MT::NC, NH = MT::NH, NT = MT::NT, QS = MT::NPL, RS = SM::ROW;
+  constexpr int ns = Lay<MAG>::NS, nf = Lay<MAG>::NF;
   constexpr int nv = MAG ? (GLM ? 9 : 8) : 5;
   const int tid = threadIdx.x;
   int b = blockIdx.x;
@@ -196,7 +200,6 @@ __global__ void __launch_bounds__(MT::NT, (MAG ? MT::MINB : MT::MINBH))
   const int k0 = (b / nty) * LZ;
   const int T0 = min(TX, G.n[0] - x0), T1 = min(TY, G.n[1] - y0);
   const int kend = min(k0 + LZ, G.n[2]);
-  const double ch = A.sc->ch;
   const AxisGeo& gz = G.g[2];
   auto slot = [&](int p) { return (p - k0 + 2) % 3; };
 
@@ -207,34 +210,32 @@ __global__ void __launch_bounds__(MT::NT, (MAG ? MT::MINB : MT::MINBH))
   const int orr = MT::pidx(oi, oj);
   const int h = tid - NC;  // index of the other threads
 
+  // the column's slots: z slope and z flux of the plane being finished, z slope of the next
+  double *const sz = &sm.R[0][SM::SZ + (owner ? tid : 0)], *const fz = &sm.R[0][SM::FZ + (owner ? tid : 0)];
+  double* const zt = &sm.R[0][SM::ZT + (owner ? tid : 0)];
+
   // ---- prologue: planes k0-2 .. k0+2, the z slopes of k0-1 and k0, face k0-1/2
+  if (tid == 0) set_flux_const(sm.fc, A);
   for (int p = k0 - 2; p <= k0; p++)
     stage_plane<MAG, GLM, MT>(G, A, sm.W[slot(p)], p, p >= k0 && p < kend, x0, y0, T0, T1, tid, NT);
   __syncthreads();
-  double szn[NS];  // the z slope of the plane above the one being finished
-  if (live)
-    slopes_to<MAG, LIM, QS>(&sm.W[slot(k0 - 2)][0][orr], &sm.W[slot(k0 - 1)][0][orr], &sm.W[slot(k0)][0][orr], gz,
-                            k0 - 1, szn, 1);
+  if (live)  // the slope of k0-1 is the face's left slope
+    slopes_to<MAG, LIM, QS, RS>(&sm.W[slot(k0 - 2)][0][orr], &sm.W[slot(k0 - 1)][0][orr], &sm.W[slot(k0)][0][orr], gz,
+                                G.n[2], k0 - 1, sz);
   __syncthreads();
   stage_plane<MAG, GLM, MT>(G, A, sm.W[slot(k0 + 1)], k0 + 1, k0 + 1 < kend, x0, y0, T0, T1, tid, NT);
   __syncthreads();
   if (live) {
-#pragma unroll
-    for (int q = 0; q < Lay<MAG>::NS; q++) sm.SZ[q][tid] = szn[q];  // the slope of k0-1 is the face's left slope
-    double szk[NS];
-    slopes_to<MAG, LIM, QS>(&sm.W[slot(k0 - 1)][0][orr], &sm.W[slot(k0)][0][orr], &sm.W[slot(k0 + 1)][0][orr], gz,
-                            k0, szk, 1);
-    double fz[9];
-    if (!z_face<MAG, MT>(&sm.W[slot(k0 - 1)][0][orr], &sm.W[slot(k0)][0][orr], sm, tid, szk, gz, k0 - 1, A, ch, fz))
+    slopes_to<MAG, LIM, QS, RS>(&sm.W[slot(k0 - 1)][0][orr], &sm.W[slot(k0)][0][orr], &sm.W[slot(k0 + 1)][0][orr], gz,
+                                G.n[2], k0, zt);
+    if (!z_face<MAG, MT>(&sm.W[slot(k0 - 1)][0][orr], &sm.W[slot(k0)][0][orr], sz, zt, gz, k0 - 1, &sm.fc, fz))
       record_error(A.sc, kENEG_EINT, x0 + oi, y0 + oj, k0 - 1);
     if (k0 == 0 && G.fb != nullptr) {  // boundary code 10 at the inner z face (fluxboundary.f90:42-87)
 #pragma unroll
-      for (int q = 0; q < Lay<MAG>::NF; q++) fz[q] = G.fb[q];
+      for (int q = 0; q < nf; q++) fz[q * RS] = G.fb[q];
     }
 #pragma unroll
-    for (int q = 0; q < Lay<MAG>::NS; q++) sm.SZ[q][tid] = szk[q];
-#pragma unroll
-    for (int q = 0; q < Lay<MAG>::NF; q++) sm.FZ[q][tid] = fz[q];
+    for (int q = 0; q < ns; q++) sz[q * RS] = zt[q * RS];
   }
   __syncthreads();
   stage_plane<MAG, GLM, MT>(G, A, sm.W[slot(k0 + 2)], k0 + 2, k0 + 2 < kend, x0, y0, T0, T1, tid, NT);
@@ -272,10 +273,9 @@ __global__ void __launch_bounds__(MT::NT, (MAG ? MT::MINB : MT::MINBH))
     // ---- phase 1: slopes --------------------------------------------------------
     // owners: the z slope of their column, then one x-y slope cell each (the
     // last NC of the list); the other threads: the rest of the list
-    if (live) slopes_to<MAG, LIM, QS>(Wk + orr, Wk1 + orr, Wk2 + orr, gz, k + 1, szn, 1);
-    constexpr int NSO = MT::OXY ? MT::NSXY - NC : MT::NSXY;  // items the other threads take
-    for (int w = owner ? (MT::OXY ? NSO + tid : MT::NSXY) : h; w < (owner ? MT::NSXY : NSO);
-         w += owner ? NC : NH) {
+    if (live) slopes_to<MAG, LIM, QS, RS>(Wk + orr, Wk1 + orr, Wk2 + orr, gz, G.n[2], k + 1, zt);
+    constexpr int NSO = MT::NSXY - NC;  // items the other threads take
+    for (int w = owner ? NSO + tid : h; w < (owner ? MT::NSXY : NSO); w += owner ? NC : NH) {
       int ax, si, sj;
       if (w < MT::NSX) {
         ax = 0;
@@ -291,8 +291,8 @@ __global__ void __launch_bounds__(MT::NT, (MAG ? MT::MINB : MT::MINBH))
       const int r = MT::pidx(si, sj);
       const int rm = ax == 0 ? MT::pidx(si - 1, sj) : MT::pidx(si, sj - 1);
       const int rp = ax == 0 ? MT::pidx(si + 1, sj) : MT::pidx(si, sj + 1);
-      slopes_to<MAG, LIM, QS>(Wk + rm, Wk + r, Wk + rp, G.g[ax], ax == 0 ? x0 + si : y0 + sj, &sm.S[0][w],
-                              MT::NSXY);
+      slopes_to<MAG, LIM, QS, RS>(Wk + rm, Wk + r, Wk + rp, G.g[ax], G.n[ax], ax == 0 ? x0 + si : y0 + sj,
+                                  &sm.R[0][SM::XY + w]);
     }
     __syncthreads();
     // ---- phase 2: face fluxes -------------------------------------------------
@@ -300,23 +300,22 @@ __global__ void __launch_bounds__(MT::NT, (MAG ? MT::MINB : MT::MINBH))
     // the z flux difference is then done before the x-y face call)
     double dz[9];
     if (live) {
-      double fz[9];
-      if (!z_face<MAG, MT>(Wk + orr, Wk1 + orr, sm, tid, szn, gz, k, A, ch, fz))
+      if (!z_face<MAG, MT>(Wk + orr, Wk1 + orr, sz, zt, gz, k, &sm.fc, sz))
         record_error(A.sc, kENEG_EINT, x0 + oi, y0 + oj, k);
       const double idz = gz.idxi[k + 2];
 #pragma unroll
-      for (int q = 0; q < Lay<MAG>::NF; q++) {
-        dz[q] = idz * (sm.FZ[q][tid] - fz[q]);
-        sm.FZ[q][tid] = fz[q];
+      for (int q = 0; q < nf; q++) {
+        const double f = sz[q * RS];
+        dz[q] = idz * (fz[q * RS] - f);
+        fz[q * RS] = f;
       }
 #pragma unroll
-      for (int q = 0; q < Lay<MAG>::NS; q++) sm.SZ[q][tid] = szn[q];
+      for (int q = 0; q < ns; q++) sz[q * RS] = zt[q * RS];
     }
     // owners, then: one x-y face each (the last NC of the list); the other
     // threads: the rest of the list
-    constexpr int NFO = MT::OXY ? MT::NFXY - NC : MT::NFXY;
-    for (int w = owner ? (MT::OXY ? NFO + tid : MT::NFXY) : h; w < (owner ? MT::NFXY : NFO);
-         w += owner ? NC : NH) {
+    constexpr int NFO = MT::NFXY - NC;
+    for (int w = owner ? NFO + tid : h; w < (owner ? MT::NFXY : NFO); w += owner ? NC : NH) {
       int ax, fi, fj, sL, sR, rL, rR, gL;
       if (w < MT::NFX) {
         ax = 0;
@@ -343,15 +342,9 @@ __global__ void __launch_bounds__(MT::NT, (MAG ? MT::MINB : MT::MINBH))
       }
       const AxisGeo& g = G.g[ax];
       const double dx1 = g.hr[gL + 2], dx2 = g.hl[gL + 3];
-      const int cn = ax, c1 = ax + 1, c2 = (ax + 2) % 3;
-      const double* PL = Wk + rL;
-      const double* PR = Wk + rR;
-      const double* SLp = &sm.S[0][sL];
-      const double* SRp = &sm.S[0][sR];
-      constexpr int SS = MT::NSXY;
-      // the flux goes straight into its conserved slots of F (put_flux)
-      if (!face_flux_fast<MAG, QS>(PL, PR, SLp, SS, SRp, SS, dx1, dx2, cn, c1, c2, A.gamma, A.gm1, ch, &sm.F[0][w],
-                                   MT::NFXY)) {
+      // the flux goes straight into its conserved slots (put_flux)
+      if (!face_flux_fast<MAG, QS, RS, RS>(Wk + rL, Wk + rR, &sm.R[0][SM::XY + sL], &sm.R[0][SM::XY + sR], dx1, dx2, ax,
+                                           &sm.fc, &sm.R[0][SM::FXY + w])) {
         int gi[3] = {x0 + fi, y0 + fj, k};
         gi[ax] = gL;
         record_error(A.sc, kENEG_EINT, gi[0], gi[1], gi[2]);
@@ -365,12 +358,12 @@ __global__ void __launch_bounds__(MT::NT, (MAG ? MT::MINB : MT::MINBH))
         const size_t c = cidx(G, i, j, k);
         double acc[9];
         const double idx1 = G.g[0].idxi[i + 2], idx2 = G.g[1].idxi[j + 2];
-        const int xm = oi + (TX + 1) * oj, ym = MT::NFX + oi + TX * oj;
+        const int xm = SM::FXY + oi + (TX + 1) * oj, ym = SM::FXY + MT::NFX + oi + TX * oj;
 #pragma unroll
         for (int q = 0; q < nv; q++) {
           acc[q] = 0.0;
-          acc[q] = acc[q] + idx1 * (sm.F[q][xm] - sm.F[q][xm + 1]);
-          acc[q] = acc[q] + idx2 * (sm.F[q][ym] - sm.F[q][ym + TX]);
+          acc[q] = acc[q] + idx1 * (sm.R[q][xm] - sm.R[q][xm + 1]);
+          acc[q] = acc[q] + idx2 * (sm.R[q][ym] - sm.R[q][ym + TX]);
           acc[q] = acc[q] + dz[q];
         }
         if (A.gphi != nullptr) cart_gravity(G, A, c, i, j, k, acc);
@@ -425,7 +418,7 @@ __global__ void __launch_bounds__(MT::NT, (MAG ? MT::MINB : MT::MINBH))
 // are short and wait on latency and barriers, and the layout takes 66 KB
 // instead of 111: three CTAs per SM at 80 registers (the 160^3 polytrope, 8
 // steps with copies: 56.1 -> 51.1 ms).
-using MT168 = March<16, 8, 128, 2, true, 3>;
+using MT168 = March<16, 8, 128, 2, 3>;
 
 template <bool MAG, bool GLM, int LIM, bool PUSH, class MT>
 cudaError_t launch_mt(const GridDev& G, const StageArgs& A, int LZ, int ntx, int nty, int nch, cudaStream_t st) {

@@ -134,14 +134,15 @@ __device__ __forceinline__ T get_cf(T d, T cs, T b1, T b2, T b3) {
 // of the normal field and phi (hlldflux.f90:19-150), then the flux of the
 // selected state (fstar, hlldflux.f90:156-179).  f[0..8] = mass, normal and
 // two tangential momenta, energy, phi-flux (normal B), two tangential B,
-// ch^2*B_n.  T = double in the FP64 path; the mixed-precision path
+// ch^2*B_n.  rch = 1/ch, correctly rounded (the same for every face of a
+// launch).  T = double in the FP64 path; the mixed-precision path
 // instantiates it for float.
 template <typename T, class D>
 __device__ __forceinline__ void hlld(T f[9], T cfl, T cfr, T v1l, T v1r, T v2l, T v2r, T v3l, T v3r, T dl, T dr, T el,
                                      T er, T ptl, T ptr, T b1l, T b1r, T b2l, T b2r, T b3l, T b3r, T phil, T phir,
-                                     T ch, D& dvp) {
+                                     T ch, T rch, D& dvp) {
   const T h = T(0.5), one = T(1.0), zero = T(0.0);
-  const T b1 = h * ((b1l + b1r) - dvp.div(phir - phil, ch, dvp.rec(ch)));
+  const T b1 = h * ((b1l + b1r) - dvp.div(phir - phil, ch, rch));
   const T phi = h * ((phil + phir) - (b1r - b1l) * ch);
   const T sl = fmin2(fmin2(v1r - cfr, v1l - cfl), zero);
   const T sr = fmax2(fmax2(v1r + cfr, v1l + cfl), zero);
@@ -268,7 +269,7 @@ __device__ __forceinline__ void hlld(T f[9], T cfl, T cfr, T v1l, T v1r, T v2l, 
                                      T ch) {
   PlainDiv dv;
   hlld(f, cfl, cfr, v1l, v1r, v2l, v2r, v3l, v3r, dl, dr, el, er, ptl, ptr, b1l, b1r, b2l, b2r, b3l, b3r, phil, phir, ch,
-       dv);
+       ch, dv);
 }
 
 }  // namespace hmn

@@ -21,20 +21,20 @@ struct SmemT {
   double S[Lay<MAG>::NS + TL::SP][TL::NSB];
   double F[Lay<MAG>::NF + TL::SP][TL::NFB];
   uint64_t bar;                   // completion barrier of the region's bulk copies
+  FluxConst fc;
 };
 
 // One axis of the fused stage: slopes, face fluxes, flux divergence of the
 // thread's own cell added to acc[].
 template <int AX, bool MAG, bool GLM, class TL, bool SPH = false>
 __device__ __forceinline__ void axis_pass(const GridDev& G, const StageArgs& A, SmemT<TL, MAG>& sm, const int t0[3],
-                                          const int T[3], double acc[9], double accs[], double ch) {
+                                          const int T[3], double acc[9], double accs[]) {
   constexpr int TX = TL::TX, TY = TL::TY, TZ = TL::TZ;
   constexpr int SBX = TX + (AX == 0 ? 2 : 0), SBY = TY + (AX == 1 ? 2 : 0), SBZ = TZ + (AX == 2 ? 2 : 0);
   constexpr int FBX = TX + (AX == 0 ? 1 : 0), FBY = TY + (AX == 1 ? 1 : 0), FBZ = TZ + (AX == 2 ? 1 : 0);
   constexpr int NSB = SBX * SBY * SBZ, NFB = FBX * FBY * FBZ;
   constexpr int SSTR = AX == 0 ? 1 : (AX == 1 ? SBX : SBX * SBY);
   constexpr int FSTR = AX == 0 ? 1 : (AX == 1 ? FBX : FBX * FBY);
-  constexpr int cn = AX, c1 = (AX + 1) % 3, c2 = (AX + 2) % 3;
   const AxisGeo& g = G.g[AX];
   const int tid = threadIdx.x;
 
@@ -54,11 +54,11 @@ __device__ __forceinline__ void axis_pass(const GridDev& G, const StageArgs& A, 
     const int cg = lc[AX] + t0[AX];  // global coordinate along AX
     // the slopes go straight to their shared-memory slots (rows of S)
     if (A.limiter == 1)
-      slopes_to<MAG, 1, TL::NR>(&sm.P[0][rm], &sm.P[0][r], &sm.P[0][rp], g, cg, &sm.S[0][w], TL::NSB);
+      slopes_to<MAG, 1, TL::NR, TL::NSB>(&sm.P[0][rm], &sm.P[0][r], &sm.P[0][rp], g, G.n[AX], cg, &sm.S[0][w]);
     else if (A.limiter == 2)
-      slopes_to<MAG, 2, TL::NR>(&sm.P[0][rm], &sm.P[0][r], &sm.P[0][rp], g, cg, &sm.S[0][w], TL::NSB);
+      slopes_to<MAG, 2, TL::NR, TL::NSB>(&sm.P[0][rm], &sm.P[0][r], &sm.P[0][rp], g, G.n[AX], cg, &sm.S[0][w]);
     else
-      slopes_to<MAG, 0, TL::NR>(&sm.P[0][rm], &sm.P[0][r], &sm.P[0][rp], g, cg, &sm.S[0][w], TL::NSB);
+      slopes_to<MAG, 0, TL::NR, TL::NSB>(&sm.P[0][rm], &sm.P[0][r], &sm.P[0][rp], g, G.n[AX], cg, &sm.S[0][w]);
     // passive-scalar slopes (interpolation.f90:135-141), not zeroed by the eint check
     if constexpr (TL::SP > 0) {
       for (int n = 0; n < A.nspc; n++) {
@@ -94,8 +94,8 @@ __device__ __forceinline__ void axis_pass(const GridDev& G, const StageArgs& A, 
     const double dx2 = g.hl[gL + 3];  // x(i+1)-xi(i)
     // the flux goes straight into its conserved slots of F (put_flux:
     // numflux.f90:186-198, 359-371, 531-543)
-    if (!face_flux_fast<MAG, TL::NR>(&sm.P[0][rL], &sm.P[0][rR], &sm.S[0][sL], TL::NSB, &sm.S[0][sR], TL::NSB, dx1,
-                                     dx2, cn, c1, c2, A.gamma, A.gm1, ch, &sm.F[0][w], TL::NFB)) {
+    if (!face_flux_fast<MAG, TL::NR, TL::NSB, TL::NFB>(&sm.P[0][rL], &sm.P[0][rR], &sm.S[0][sL], &sm.S[0][sR], dx1,
+                                                       dx2, AX, &sm.fc, &sm.F[0][w])) {
       int gi[3] = {t0[0] + fx, t0[1] + fy, t0[2] + fz};
       gi[AX] = gL;
       record_error(A.sc, kENEG_EINT, gi[0], gi[1], gi[2]);  // numflux.f90:117 -> error_flux
@@ -197,6 +197,7 @@ __device__ __forceinline__ void stage_tile_exact(const GridDev& G, const StageAr
   // Every slot of the full-tile layout is one local cell (pidx and
   // region_cell are inverse); a ragged tile needs the cells within two of
   // its real extent, so its high halo occupies interior-layout slots.
+  if (tid == 0) set_flux_const(sm.fc, A);
   stage_region<MAG, GLM, TL>(G, A, sm.P, &sm.bar, tm, t0, T);
 
   double acc[9];
@@ -205,10 +206,9 @@ __device__ __forceinline__ void stage_tile_exact(const GridDev& G, const StageAr
   double accs[TL::SP > 0 ? TL::SP : 1];
 #pragma unroll
   for (int n = 0; n < (TL::SP > 0 ? TL::SP : 1); n++) accs[n] = 0.0;
-  const double ch = A.sc->ch;
-  if (TL::TX > 1 && G.solve[0]) axis_pass<0, MAG, GLM, TL, SPH>(G, A, sm, t0, T, acc, accs, ch);
-  if (TL::TY > 1 && G.solve[1]) axis_pass<1, MAG, GLM, TL, SPH>(G, A, sm, t0, T, acc, accs, ch);
-  if (TL::TZ > 1 && G.solve[2]) axis_pass<2, MAG, GLM, TL, SPH>(G, A, sm, t0, T, acc, accs, ch);
+  if (TL::TX > 1 && G.solve[0]) axis_pass<0, MAG, GLM, TL, SPH>(G, A, sm, t0, T, acc, accs);
+  if (TL::TY > 1 && G.solve[1]) axis_pass<1, MAG, GLM, TL, SPH>(G, A, sm, t0, T, acc, accs);
+  if (TL::TZ > 1 && G.solve[2]) axis_pass<2, MAG, GLM, TL, SPH>(G, A, sm, t0, T, acc, accs);
 
   // ---- RK combination (rungekutta.f90:35-59) + source (source.f90:70-85) -------
   if (tid >= TL::NC) return;
