@@ -1521,16 +1521,17 @@ static int enqueue_step(hmn_ctx* ctx) {
 // (hmn_small.cu) instead of a chain of six launches per step.
 constexpr size_t kSmallCells = 65536;
 
-static bool small_run_ok(hmn_ctx* ctx) {
+static bool small_run_ok(hmn_ctx* ctx, int tile[3]) {
   const char* e = getenv("HMN_SMALL");  // HMN_SMALL=0 keeps the per-phase launches
   if (e && e[0] == '0') return false;
   return ctx->par.precision == 0 && ctx->par.nspc == 0 && (ctx->par.rktype == 2 || ctx->par.rktype == 3) &&
-         !ctx->zpush_on && ctx->plane <= kSmallCells && small_run_supported(ctx->tile, ctx->G.sph.on != 0);
+         !ctx->zpush_on && ctx->plane <= kSmallCells &&
+         small_run_tile(ctx->tile, ctx->n, ctx->nsm, ctx->G.sph.on != 0, tile);
 }
 
 // Up to max_steps steps of the device loop in persistent launches of at
 // most 4096 steps each; the clock, dt and end test stay on the device.
-static int run_small(hmn_ctx* ctx, int max_steps) {
+static int run_small(hmn_ctx* ctx, int max_steps, const int tile[3]) {
   for (int a = 0; a < 3; a++)
     for (int io = 0; io < 2; io++)
       if (ctx->solve[a] && (ctx->bc[a][io][0] >= 9 || ctx->bc[a][io][1] >= 9) && !ctx->G.dir[a][io])
@@ -1538,16 +1539,28 @@ static int run_small(hmn_ctx* ctx, int max_steps) {
   if (ctx->solve[2] && ctx->bc[2][0][0] == 10 && !ctx->fb) return HMN_EBADCFG;
   if (!ctx->small_bar) CK(cudaMalloc((void**)&ctx->small_bar, 2 * sizeof(unsigned int)), "barrier");
   const int rk = ctx->par.rktype;
+  int tiles[3];
+  for (int a = 0; a < 3; a++) tiles[a] = (ctx->n[a] + tile[a] - 1) / tile[a];
   SmallRun R;
   memset(&R, 0, sizeof(R));
-  for (int p = 0; p < 2; p++)
-    for (int s = 1; s <= rk; s++) R.st[p][s - 1] = stage_args(ctx, s, (ctx->pcur + p + s - 1) & 1);
+  const auto set_stages = [&](int par) {  // the stages of two steps from primitive buffer parity par on
+    for (int p = 0; p < 2; p++)
+      for (int s = 1; s <= rk; s++) {
+        StageArgs a = stage_args(ctx, s, (par + p + s - 1) & 1);
+        for (int d = 0; d < 3; d++) {
+          a.tile[d] = tile[d];
+          a.tiles[d] = tiles[d];
+        }
+        R.st[p][s - 1] = a;
+      }
+  };
+  set_stages(ctx->pcur);
   R.sc = ctx->sc;
   R.bar = ctx->small_bar;
   R.damp = ctx->glm ? std::exp(-ctx->par.alpha9wave * ctx->par.courant) : 1.0;
   R.phifac0 = ctx->phifac;
   R.rk = rk;
-  R.ntiles = ctx->tiles[0] * ctx->tiles[1] * ctx->tiles[2];
+  R.ntiles = tiles[0] * tiles[1] * tiles[2];
   const int tn0 = ctx->sc_h->tn, pcur0 = ctx->pcur;
   int left = max_steps;
   while (left > 0) {
@@ -1556,7 +1569,7 @@ static int run_small(hmn_ctx* ctx, int max_steps) {
     int grid = 0;
     // the barrier's arrival counter starts every launch at zero
     CK(cudaMemsetAsync(ctx->small_bar, 0, sizeof(unsigned int), ctx->st), "barrier");
-    CK(launch_small_run(ctx->G, R, ctx->mag != 0, ctx->glm != 0, ctx->G.sph.on != 0, ctx->tile, ctx->st, &grid),
+    CK(launch_small_run(ctx->G, R, ctx->mag != 0, ctx->glm != 0, ctx->G.sph.on != 0, tile, ctx->st, &grid),
        "small run");
     ctx->launches += 1;
     const int rc = fetch_scalars(ctx);
@@ -1567,9 +1580,7 @@ static int run_small(hmn_ctx* ctx, int max_steps) {
     const int ran = ctx->sc_h->tn - tn_before;
     if (ran > 0) R.phifac0 = R.damp;  // the next launch's first step follows a step of this one
     // the parity of the primitive buffer moves with the steps that ran
-    for (int p = 0; p < 2; p++)
-      for (int s = 1; s <= rk; s++)
-        R.st[p][s - 1] = stage_args(ctx, s, (pcur0 + rk * (ctx->sc_h->tn - tn0) + p + s - 1) & 1);
+    set_stages(pcur0 + rk * (ctx->sc_h->tn - tn0));
     if (ctx->sc_h->err_code || ctx->sc_h->done || ran < R.nsteps) break;
     left -= R.nsteps;
   }
@@ -1644,8 +1655,9 @@ extern "C" int hmn_run(hmn_ctx* ctx, double* time, double t_end, int max_steps, 
   if (rc) return rc;
   const int tn0 = ctx->sc_h->tn;
   const int pcur0 = ctx->pcur;
-  if (small_run_ok(ctx)) {
-    rc = run_small(ctx, max_steps);
+  int small_tile[3];
+  if (small_run_ok(ctx, small_tile)) {
+    rc = run_small(ctx, max_steps, small_tile);
     if (rc) return rc;
     *time = ctx->sc_h->time;
     if (steps) *steps = ctx->sc_h->tn - tn0;

@@ -207,7 +207,7 @@ bool march_enabled();
 void march_chunks(const int n[3], int* lz, int* ntx, int* nty, int* nch);
 // up to R.nsteps steps of a small grid in one cooperative launch of at most
 // one CTA per tile (hmn_small.cu); *grid receives the CTA count
-int small_run_supported(const int tile[3], bool sph);
+int small_run_tile(const int tile[3], const int n[3], int nsm, bool sph, int out[3]);
 cudaError_t launch_small_run(const GridDev& G, const SmallRun& R, bool mag, bool glm, bool sph, const int tile[3],
                              cudaStream_t st, int* grid);
 // mixed precision (hmn_mixed.cu): FP32 Riemann solver, FP64 reconstruction and accumulation

@@ -170,25 +170,66 @@ cudaError_t launch_mag(const GridDev& G, const SmallRun& R, bool mag, bool glm, 
 
 }  // namespace
 
-int small_run_supported(const int tile[3], bool sph) {
-  if (tile[0] == 256 && tile[1] == 1 && tile[2] == 1) return 1;
-  if (tile[0] == 16 && tile[1] == 16 && tile[2] == 1) return 1;
-  if (tile[0] == 8 && tile[1] == 8 && tile[2] == 8) return sph ? 0 : 1;
-  return 0;
+// The tiles of the persistent loop, by the grid's solved axes (those of the
+// stage tile).  A step is a chain of phases, each as long as one CTA's slopes,
+// faces and cells take, and that grows with the warps that share an SM.  So
+// the grid is cut into the smallest tiles that still give (about) every SM no
+// more than one CTA of the next size up: 1-D tiles of 30 cells are one warp
+// (32 slope cells), and their barriers cost nothing.  The larger tiles compute
+// fewer halo slopes and faces twice and stay for the larger grids.
+// Against the largest tiles throughout: 128x128 MHD, 64 steps 3.84 -> 3.00 ms;
+// 500 radial cells, 64 steps 1.79 -> 1.65 ms.
+static int tiles_of(const int n[3], const int t[3]) {
+  int c = 1;
+  for (int a = 0; a < 3; a++) c *= (n[a] + t[a] - 1) / t[a];
+  return c;
+}
+
+int small_run_tile(const int tile[3], const int n[3], int nsm, bool sph, int out[3]) {
+  static const int one[3][3] = {{30, 1, 1}, {126, 1, 1}, {256, 1, 1}};
+  static const int two[3][3] = {{8, 8, 1}, {16, 8, 1}, {16, 16, 1}};
+  static const int three[2][3] = {{8, 4, 4}, {8, 8, 8}};
+  const int(*t)[3] = nullptr;
+  int kinds = 3;
+  if (tile[0] == 256 && tile[1] == 1 && tile[2] == 1) t = one;
+  if (tile[0] == 16 && tile[1] == 16 && tile[2] == 1) t = two;
+  if (tile[0] == 8 && tile[1] == 8 && tile[2] == 8 && !sph) t = three, kinds = 2;
+  if (t == nullptr) return 0;
+  int k = 0;
+  while (k + 1 < kinds && tiles_of(n, t[k]) > (k == 0 ? 1 : 2) * nsm) k++;
+  for (int a = 0; a < 3; a++) out[a] = t[k][a];
+  return 1;
 }
 
 cudaError_t launch_small_run(const GridDev& G, const SmallRun& R, bool mag, bool glm, bool sph, const int tile[3],
                              cudaStream_t st, int* grid) {
-  if (tile[0] == 256 && tile[1] == 1 && tile[2] == 1) {
-    if (sph) return launch_mag<Tile<256, 1, 1, 288, 2>, true>(G, R, mag, glm, st, grid);
-    return launch_mag<Tile<256, 1, 1, 288, 2>, false>(G, R, mag, glm, st, grid);
+  const int t = tile[0] * 10000 + tile[1] * 100 + tile[2];
+  switch (t) {
+    case 300101:
+      return sph ? launch_mag<Tile<30, 1, 1, 32, 2>, true>(G, R, mag, glm, st, grid)
+                 : launch_mag<Tile<30, 1, 1, 32, 2>, false>(G, R, mag, glm, st, grid);
+    case 1260101:
+      return sph ? launch_mag<Tile<126, 1, 1, 128, 2>, true>(G, R, mag, glm, st, grid)
+                 : launch_mag<Tile<126, 1, 1, 128, 2>, false>(G, R, mag, glm, st, grid);
+    case 2560101:
+      return sph ? launch_mag<Tile<256, 1, 1, 288, 2>, true>(G, R, mag, glm, st, grid)
+                 : launch_mag<Tile<256, 1, 1, 288, 2>, false>(G, R, mag, glm, st, grid);
+    case 80801:
+      return sph ? launch_mag<Tile<8, 8, 1, 96, 2>, true>(G, R, mag, glm, st, grid)
+                 : launch_mag<Tile<8, 8, 1, 96, 2>, false>(G, R, mag, glm, st, grid);
+    case 160801:
+      return sph ? launch_mag<Tile<16, 8, 1, 160, 2>, true>(G, R, mag, glm, st, grid)
+                 : launch_mag<Tile<16, 8, 1, 160, 2>, false>(G, R, mag, glm, st, grid);
+    case 161601:
+      return sph ? launch_mag<Tile<16, 16, 1, 288, 2>, true>(G, R, mag, glm, st, grid)
+                 : launch_mag<Tile<16, 16, 1, 288, 2>, false>(G, R, mag, glm, st, grid);
+    case 80404:
+      if (!sph) return launch_mag<Tile<8, 4, 4, 192, 2>, false>(G, R, mag, glm, st, grid);
+      break;
+    case 80808:
+      if (!sph) return launch_mag<Tile<8, 8, 8, 640, 1>, false>(G, R, mag, glm, st, grid);
+      break;
   }
-  if (tile[0] == 16 && tile[1] == 16 && tile[2] == 1) {
-    if (sph) return launch_mag<Tile<16, 16, 1, 288, 2>, true>(G, R, mag, glm, st, grid);
-    return launch_mag<Tile<16, 16, 1, 288, 2>, false>(G, R, mag, glm, st, grid);
-  }
-  if (tile[0] == 8 && tile[1] == 8 && tile[2] == 8 && !sph)
-    return launch_mag<Tile<8, 8, 8, 640, 1>, false>(G, R, mag, glm, st, grid);
   return cudaErrorNotSupported;
 }
 
