@@ -36,12 +36,18 @@ struct SlotInfo {
 
 struct Klass {
   int kind;
+  int tile;          // the schedule's tile of its kind, or that of a class of few items
+  bool few;          // the latter: the last stage reduces the CFL quantities too
   bool mag, glm;
   int first, count;  // range in the item list
   int grid;          // persistent CTAs of the stage launches
   bool dynamic;      // stage launches take items from the shared counter
   int* queue;        // that counter: {next item, CTAs finished}
 };
+
+// Steps captured in one graph: between two replays the GPU idles a few
+// microseconds, a tenth of a step of small grids.
+constexpr int kManySteps = 8;
 
 constexpr int kMaxClasses = 9;  // three tile kinds x (hydro, MHD, MHD with GLM)
 
@@ -63,6 +69,7 @@ struct hmn_batch {
   int2* d_items = nullptr;
   size_t items_cap = 0;
   std::vector<Klass> classes;
+  int listed = 0;  // simulations in the work list
   bool dirty = true;
   cudaStream_t st = nullptr;
   int nsm = 148;
@@ -72,11 +79,18 @@ struct hmn_batch {
   int* d_queue = nullptr;             // one counter pair per class: classes run side by side
   cudaStream_t side[kMaxClasses] = {};  // branches of the captured step beside st (classes 1, 2, ...)
   cudaEvent_t fork = nullptr, join[kMaxClasses] = {};
-  cudaGraphExec_t graph = nullptr;
+  cudaGraphExec_t graph = nullptr, graph_many = nullptr;  // one step; kManySteps steps
+  long long step_launches = 0;        // kernel launches of one step
   long long launches = 0;
   double* stage_h = nullptr;
   size_t stage_h_bytes = 0;
 };
+
+static void drop_graphs(hmn_batch* b) {
+  if (b->graph) cudaGraphExecDestroy(b->graph);
+  if (b->graph_many) cudaGraphExecDestroy(b->graph_many);
+  b->graph = b->graph_many = nullptr;
+}
 
 static int cuda_fail(cudaError_t e, const char* what) {
   if (e == cudaSuccess) return HMN_OK;
@@ -169,7 +183,7 @@ extern "C" int hmn_batch_create(size_t pool_bytes, int max_sims, int precision, 
 extern "C" int hmn_batch_destroy(hmn_batch* b) {
   if (!b) return HMN_EINVAL;
   if (b->st) cudaStreamSynchronize(b->st);
-  if (b->graph) cudaGraphExecDestroy(b->graph);
+  drop_graphs(b);
   cudaFree(b->pool);
   cudaFree(b->d_sims);
   cudaFree(b->d_items);
@@ -409,6 +423,12 @@ extern "C" int hmn_batch_set_held(hmn_batch* b, const int* held) {
   return HMN_OK;
 }
 
+static int start_steps(hmn_batch* b);
+
+static int tiles_of(const int n[3], const int t[3]) {
+  return ((n[0] + t[0] - 1) / t[0]) * ((n[1] + t[1] - 1) / t[1]) * ((n[2] + t[2] - 1) / t[2]);
+}
+
 static int rebuild(hmn_batch* b) {
   // work list: active, unfinished simulations grouped by (tile kind, mag, glm)
   std::vector<int2> items;
@@ -417,34 +437,58 @@ static int rebuild(hmn_batch* b) {
     for (int m = 0; m < 3; m++) {
       const bool mag = m > 0, glm = m == 2;
       const int sweep = b->sweep[kind];
-      Klass k{kind, mag, glm, (int)items.size(), 0, 0, sweep == HMN_SWEEP_DYNAMIC, nullptr};
+      Klass k{kind, b->tile_id[kind], false, mag, glm, (int)items.size(), 0, 0, sweep == HMN_SWEEP_DYNAMIC, nullptr};
       std::vector<int> sims;
-      int most = 0;
+      int most_tiles = 0;
       for (int s = 0; s < b->max_sims; s++) {
         const SlotInfo& si = b->slots[s];
         if (!si.used || si.kind != kind || si.mag != mag || si.glm != glm || b->h_sims[s].sc.done ||
             b->h_sims[s].held)
           continue;
         sims.push_back(s);
-        most = std::max(most, si.ntiles);
+        most_tiles = std::max(most_tiles, si.ntiles);
+      }
+      // items of each listed simulation: the schedule's tiles, or smaller ones
+      // where those are few (FP64)
+      std::vector<int> ntiles(b->max_sims, 0);
+      for (int s : sims) ntiles[s] = b->slots[s].ntiles;
+      if (b->precision == 0 && !sims.empty()) {
+        int most, few[3];
+        const int id = batch_few_tile(kind, b->nsm, &most);
+        batch_tile_shape(id, few);
+        long long count = 0;
+        for (int s : sims) count += tiles_of(b->slots[s].n, few);
+        if (count <= most) {
+          k.few = true;
+          k.tile = id;
+          k.dynamic = false;
+          most_tiles = 0;
+          for (int s : sims) {
+            ntiles[s] = tiles_of(b->slots[s].n, few);
+            most_tiles = std::max(most_tiles, ntiles[s]);
+          }
+        }
       }
       if (sweep == HMN_SWEEP_INTERLEAVED) {  // tile t of every simulation, then tile t + 1
-        for (int t = 0; t < most; t++)
+        for (int t = 0; t < most_tiles; t++)
           for (int s : sims)
-            if (t < b->slots[s].ntiles) items.push_back(make_int2(s, t));
+            if (t < ntiles[s]) items.push_back(make_int2(s, t));
       } else {
         if (sweep == HMN_SWEEP_DYNAMIC)  // the largest simulations first
           std::stable_sort(sims.begin(), sims.end(),
                            [b](int x, int y) { return b->slots[x].ntiles > b->slots[y].ntiles; });
         for (int s : sims)
-          for (int t = 0; t < b->slots[s].ntiles; t++) items.push_back(make_int2(s, t));
+          for (int t = 0; t < ntiles[s]; t++) items.push_back(make_int2(s, t));
       }
       k.count = (int)items.size() - k.first;
       if (k.count) {
         // occupancy queries run here, outside any stream capture
         int per = b->blocks_per_sm[kind];
-        if (per <= 0) per = batch_stage_blocks_per_sm(b->tile_id[kind], mag, glm, b->precision);
-        k.grid = (int)std::min<long long>((long long)per * b->nsm, k.count);
+        if (k.few)
+          BCK(launch_batch_stage(b->d_sims, nullptr, 0, k.tile, mag, glm, 1, b->rktype, 0, 0, nullptr, b->st), "stage");
+        else if (per <= 0)
+          per = batch_stage_blocks_per_sm(b->tile_id[kind], mag, glm, b->precision);
+        k.grid = k.few ? k.count : (int)std::min<long long>((long long)per * b->nsm, k.count);
         k.queue = b->d_queue + 2 * b->classes.size();
         b->classes.push_back(k);
       }
@@ -459,10 +503,10 @@ static int rebuild(hmn_batch* b) {
     BCK(cudaMemcpyAsync(b->d_items, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice, b->st),
         "items");
   BCK(cudaStreamSynchronize(b->st), "sync");
-  if (b->graph) {
-    cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
-  }
+  drop_graphs(b);
+  b->listed = 0;
+  for (const Klass& k : b->classes)
+    for (int i = 0; i < k.count; i++) b->listed += items[(size_t)k.first + i].y == 0;
   // the branches of the captured step, made outside any capture
   if (b->classes.size() > 1 && !b->fork)
     BCK(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming), "fork event");
@@ -471,7 +515,7 @@ static int rebuild(hmn_batch* b) {
     if (!b->join[c]) BCK(cudaEventCreateWithFlags(&b->join[c], cudaEventDisableTiming), "join event");
   }
   b->dirty = false;
-  return HMN_OK;
+  return start_steps(b);
 }
 
 // Run f(class, stream) for every class: the first on the batch's stream, the
@@ -491,34 +535,73 @@ static int for_each_class(hmn_batch* b, F&& f) {
   return rc;
 }
 
-// One step of every listed simulation.  A simulation is in one class and the
-// launches of a class touch nothing of another's simulations, so the classes
-// run side by side, as branches of the captured graph: a served stream of
-// small 1-D, 2-D and 3-D grids waits on latency, and its step is as long as
-// the slowest class instead of their sum (24 requests 1.00 -> 0.89 s).
-static int enqueue_step(hmn_batch* b, long long* nlaunch) {
-  int rc = for_each_class(b, [&](const Klass& k, cudaStream_t st) {
-    BCK(launch_batch_cfl(b->d_sims, b->d_items + k.first, k.count, b->tile_id[k.kind], k.mag,
-                         std::min(k.count, b->nsm * 4), st),
-        "batch cfl");
-    (*nlaunch)++;
-    return (int)HMN_OK;
-  });
-  if (rc) return rc;
+static int enqueue_cfl(hmn_batch* b, const Klass& k, int after, cudaStream_t st) {
+  BCK(launch_batch_cfl(b->d_sims, b->d_items + k.first, k.count, k.tile, k.mag, after, std::min(k.count, b->nsm * 4),
+                       st),
+      "batch cfl");
+  return HMN_OK;
+}
+
+// dt of the listed simulations' current states; every step then ends with the
+// next one's.  (For a simulation that has stepped before it is the dt that its
+// last step left, formed again from the same state.)
+static int start_steps(hmn_batch* b) {
+  if (b->classes.empty()) return HMN_OK;
+  for (const Klass& k : b->classes) {
+    const int rc = enqueue_cfl(b, k, 0, b->st);
+    if (rc) return rc;
+  }
   BCK(launch_batch_finalize(b->d_sims, b->max_sims, b->st), "batch finalize");
-  (*nlaunch)++;
-  rc = for_each_class(b, [&](const Klass& k, cudaStream_t st) {
+  b->launches += (long long)b->classes.size() + 1;
+  return HMN_OK;
+}
+
+// One step of every listed simulation: its RK stages, the CFL reduction of the
+// new state, and the advance of the clocks with the next dt.  A simulation is
+// in one class and the launches of a class touch nothing of another's
+// simulations, so the classes run side by side, as branches of the captured
+// graph: a served stream of small 1-D, 2-D and 3-D grids waits on latency, and
+// its step is as long as the slowest class instead of their sum (24 requests
+// 1.00 -> 0.89 s).  With the tiles of classes of few items, the reduction in
+// their last stage, the clocks' two kernels in one and several steps per graph
+// the same stream takes 0.67 s.
+static int enqueue_step(hmn_batch* b, long long* nlaunch) {
+  const int rc = for_each_class(b, [&](const Klass& k, cudaStream_t st) {
     for (int s = 1; s <= b->rktype; s++) {
-      BCK(launch_batch_stage(b->d_sims, b->d_items + k.first, k.count, b->tile_id[k.kind], k.mag, k.glm, s, b->rktype,
+      BCK(launch_batch_stage(b->d_sims, b->d_items + k.first, k.count, k.tile, k.mag, k.glm, s, b->rktype,
                              b->precision, k.grid, k.dynamic ? k.queue : nullptr, st),
           "batch stage");
       (*nlaunch)++;
     }
-    return (int)HMN_OK;
+    if (k.few) return (int)HMN_OK;
+    (*nlaunch)++;
+    return enqueue_cfl(b, k, b->rktype, st);
   });
   if (rc) return rc;
   BCK(launch_batch_advance(b->d_sims, b->max_sims, b->st), "batch advance");
   (*nlaunch)++;
+  return HMN_OK;
+}
+
+// `steps` steps as one graph; replaying it advances every simulation by that many
+static int capture_steps(hmn_batch* b, int steps, cudaGraphExec_t* out) {
+  cudaGraph_t g;
+  BCK(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal), "capture");
+  int rc = HMN_OK;
+  for (int s = 0; s < steps && rc == HMN_OK; s++) {
+    b->step_launches = 0;
+    rc = enqueue_step(b, &b->step_launches);
+  }
+  cudaError_t e = cudaStreamEndCapture(b->st, &g);
+  if (rc) {
+    if (e == cudaSuccess) cudaGraphDestroy(g);
+    return rc;
+  }
+  BCK(e, "capture end");
+  e = cudaGraphInstantiate(out, g, 0);
+  cudaGraphDestroy(g);
+  if (e != cudaSuccess) *out = nullptr;
+  BCK(e, "graph instantiate");
   return HMN_OK;
 }
 
@@ -531,27 +614,18 @@ extern "C" int hmn_batch_step(hmn_batch* b, int nsteps) {
     if (rc) return rc;
   }
   if (b->classes.empty() || nsteps == 0) return HMN_OK;
-  long long per_step = 0;
-  if (!b->graph) {
-    // capture one step; replaying it advances every simulation by one step
-    cudaGraph_t g;
-    BCK(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal), "capture");
-    int rc = enqueue_step(b, &per_step);
-    cudaError_t e = cudaStreamEndCapture(b->st, &g);
-    if (rc) {
-      if (e == cudaSuccess) cudaGraphDestroy(g);
-      return rc;
+  int left = nsteps;
+  while (left > 0) {
+    const int n = left >= kManySteps ? kManySteps : 1;
+    cudaGraphExec_t* g = n == 1 ? &b->graph : &b->graph_many;
+    if (!*g) {
+      const int rc = capture_steps(b, n, g);
+      if (rc) return rc;
     }
-    BCK(e, "capture end");
-    e = cudaGraphInstantiate(&b->graph, g, 0);
-    cudaGraphDestroy(g);
-    BCK(e, "graph instantiate");
-  } else {
-    // launches per step equal those of the captured sequence
-    per_step = (long long)b->classes.size() * (1 + b->rktype) + 2;
+    BCK(cudaGraphLaunch(*g, b->st), "graph launch");
+    left -= n;
   }
-  for (int s = 0; s < nsteps; s++) BCK(cudaGraphLaunch(b->graph, b->st), "graph launch");
-  b->launches += per_step * nsteps;
+  b->launches += b->step_launches * nsteps;
   return HMN_OK;
 }
 
@@ -569,17 +643,14 @@ extern "C" int hmn_batch_poll(hmn_batch* b, double* time, int* tn, int* done, in
     if (b->slots[s].used && S.sc.done) any_done = true;
   }
   // drop finished simulations from the work list at the next step: the list
-  // is rebuilt only when its tile count differs from that of the used,
-  // unfinished and not held simulations (the set rebuild() lists), so a
-  // finished simulation left in its slot does not force a rebuild and graph
-  // re-capture at every poll
+  // is rebuilt only when it lists another number of simulations than are used,
+  // unfinished and not held, so a finished simulation left in its slot does not
+  // force a rebuild and graph re-capture at every poll
   if (any_done) {
-    size_t live = 0;
-    for (const Klass& k : b->classes) live += k.count;
-    size_t want = 0;
+    int want = 0;
     for (int s = 0; s < b->max_sims; s++)
-      if (b->slots[s].used && !b->h_sims[s].sc.done && !b->h_sims[s].held) want += b->slots[s].ntiles;
-    if (want != live) b->dirty = true;
+      if (b->slots[s].used && !b->h_sims[s].sc.done && !b->h_sims[s].held) want++;
+    if (want != b->listed) b->dirty = true;
   }
   return HMN_OK;
 }
@@ -633,10 +704,7 @@ extern "C" int hmn_batch_set_schedule(hmn_batch* b, int kind, int tile_id, int b
     BCK(cudaStreamSynchronize(b->st), "sync");
   }
   b->dirty = true;
-  if (b->graph) {
-    cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
-  }
+  drop_graphs(b);
   return HMN_OK;
 }
 

@@ -241,8 +241,9 @@ cudaError_t launch_evo(const GridDev& G, const double* P, size_t plane, const do
 int batch_tile_kind(const int solve[3]);
 int batch_tile_variants(int kind, int* tile_ids);
 void batch_tile_shape(int tile_id, int tile[3]);
-cudaError_t launch_batch_cfl(SimDesc* sims, const int2* items, int nitems, int kind, bool mag, int grid,
+cudaError_t launch_batch_cfl(SimDesc* sims, const int2* items, int nitems, int tid, bool mag, int after, int grid,
                              cudaStream_t st);
+int batch_few_tile(int kind, int nsm, int* most);
 cudaError_t launch_batch_finalize(SimDesc* sims, int nsims, cudaStream_t st);
 cudaError_t launch_batch_stage(SimDesc* sims, const int2* items, int nitems, int kind, bool mag, bool glm,
                                int stage, int rk, int precision, int grid, int* queue, cudaStream_t st);

@@ -490,6 +490,10 @@ using T3D4 = Tile<8, 8, 4, 384, 2, 0, 3>;
 using T2D = Tile<16, 16, 1, 288, 3, 0, 4>;
 using T2D8 = Tile<32, 8, 1, 320, 3, 0, 4>;
 using T1D = Tile<256, 1, 1, 288, 3, 0, 4>;
+// tiles of a class that leaves most of the GPU idle (batch_few_tile)
+using F3D = Tile<8, 4, 4, 192, 1>;
+using F2D = Tile<8, 8, 1, 96, 1>;
+using F1D = Tile<30, 1, 1, 32, 1>;
 
 // tile ids: 0 3-D 8x8x8 (640 threads), 1 3-D 8x8x4 (256 threads, 2 CTAs/SM),
 // 2 2-D 16x16, 3 2-D 32x8, 4 1-D 256.  batch_tile_kind gives the grid's
@@ -519,8 +523,50 @@ int batch_tile_variants(int kind, int* ids) {
 }
 
 void batch_tile_shape(int tid, int tile[3]) {
-  const int shapes[5][3] = {{8, 8, 8}, {8, 8, 4}, {16, 16, 1}, {32, 8, 1}, {256, 1, 1}};
+  const int shapes[8][3] = {{8, 8, 8}, {8, 8, 4}, {16, 16, 1}, {32, 8, 1}, {256, 1, 1}, {8, 4, 4}, {8, 8, 1}, {30, 1, 1}};
   for (int a = 0; a < 3; a++) tile[a] = shapes[tid][a];
+}
+
+// The tile a class of few items takes instead of the schedule's (ids 5 to 7,
+// chosen inside a batch only): as in the persistent small-grid loop, a step of
+// small grids is a chain of phases as long as one CTA's work, so the class is
+// cut into small tiles as long as they leave an SM about one warp per
+// scheduler: `most` is that many items.  Their last RK stage also reduces the
+// CFL quantities of the state it writes, which a class that fills the GPU does
+// not, for it would pay for the reduction's arithmetic at the stage's occupancy.
+int batch_few_tile(int kind, int nsm, int* most) {
+  *most = (kind == 0 ? 1 : (kind == 1 ? 2 : 4)) * nsm;
+  return 5 + kind;
+}
+
+// the stage arguments of one batched simulation on this kernel's tiles
+template <class TL>
+__device__ __forceinline__ StageArgs tiled_stage_args(SimDesc& S, int stage, int rk) {
+  StageArgs A = batch_stage_args(S, stage, rk);
+  constexpr int TT[3] = {TL::TX, TL::TY, TL::TZ};
+#pragma unroll
+  for (int a = 0; a < 3; a++) A.tiles[a] = (S.G.n[a] + TT[a] - 1) / TT[a];
+  return A;
+}
+
+// One RK stage of a class of few items, one CTA per item; the last stage also
+// reduces the next step's CFL quantities (cfl_kernel's values).
+template <bool MAG, bool GLM, class TL>
+__global__ void __launch_bounds__(TL::NT, TL::MINB) batch_few_kernel(SimDesc* sims, const int2* items, int stage,
+                                                                     int rk) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  SmemT<TL, MAG>& sm = *reinterpret_cast<SmemT<TL, MAG>*>(smem_raw);
+  const int2 w = items[blockIdx.x];
+  SimDesc& S = sims[w.x];
+  if (!S.active || S.sc.done) return;
+  const StageArgs A = tiled_stage_args<TL>(S, stage, rk);
+  if (stage < rk) {
+    stage_tile_exact<MAG, GLM, TL>(S.G, A, sm, w.y, nullptr);
+    return;
+  }
+  double my_dti = __longlong_as_double(0x7ff0000000000000LL), my_cf = 0.0;
+  stage_tile_exact<MAG, GLM, TL, false, false, true>(S.G, A, sm, w.y, nullptr, &my_dti, &my_cf);
+  cfl_block_reduce(my_dti, my_cf, &S.sc);
 }
 
 template <bool MAG, bool GLM, class TL, bool DYN>
@@ -532,14 +578,16 @@ __global__ void __launch_bounds__(TL::NT, (MAG ? TL::MINB : TL::MINBH)) batch_st
     const int2 w = items[it];
     SimDesc& S = sims[w.x];
     if (!S.active || S.sc.done) return;
-    const StageArgs A = batch_stage_args(S, stage, rk);
+    const StageArgs A = tiled_stage_args<TL>(S, stage, rk);
     stage_tile_exact<MAG, GLM, TL>(S.G, A, sm, w.y, nullptr);
     __syncthreads();
   });
 }
 
+// CFL quantities of the state `after` RK stages past the current one (0: the
+// current state; rk: the state the step's last stage wrote)
 template <bool MAG, class TL>
-__global__ void __launch_bounds__(TL::NT) batch_cfl_kernel(SimDesc* sims, const int2* items, int nitems) {
+__global__ void __launch_bounds__(TL::NT) batch_cfl_kernel(SimDesc* sims, const int2* items, int nitems, int after) {
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const int2 w = items[it];
     SimDesc& S = sims[w.x];
@@ -549,13 +597,13 @@ __global__ void __launch_bounds__(TL::NT) batch_cfl_kernel(SimDesc* sims, const 
     constexpr int TT[3] = {TL::TX, TL::TY, TL::TZ};
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-      const int ti = bid % S.tiles[a];
-      bid /= S.tiles[a];
+      const int tiles = (G.n[a] + TT[a] - 1) / TT[a], ti = bid % tiles;
+      bid /= tiles;
       t0[a] = ti * TT[a];
       T[a] = min(TT[a], G.n[a] - t0[a]);
     }
     double my_dti = __longlong_as_double(0x7ff0000000000000LL), my_cf = 0.0;
-    const double* P = S.P[S.pcur];
+    const double* P = S.P[(S.pcur + after) & 1];
     for (int c = threadIdx.x; c < TL::NC; c += TL::NT) {
       const int cx = c % TL::TX, cy = (c / TL::TX) % TL::TY, cz = c / (TL::TX * TL::TY);
       if (cx >= T[0] || cy >= T[1] || cz >= T[2]) continue;
@@ -576,7 +624,8 @@ __global__ void batch_finalize_kernel(SimDesc* sims, int nsims) {
 }
 
 // time += dt, tn += 1, end check (hormone.f90:147-155); primitive buffer
-// parity and the phidamp factor (source.f90:239-260) for the next step
+// parity and the phidamp factor (source.f90:239-260) for the next step, and
+// that step's dt from the CFL quantities reduced after the last stage
 __global__ void batch_advance_kernel(SimDesc* sims, int nsims) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsims) return;
@@ -591,7 +640,13 @@ __global__ void batch_advance_kernel(SimDesc* sims, int nsims) {
     S.U[1] = t;
   }
   S.phifac = S.glm ? S.damp : 1.0;
-  if (S.sc.endstyle == 1 && S.sc.time >= S.sc.t_end) S.sc.done = 1;
+  if (S.sc.endstyle == 1 && S.sc.time >= S.sc.t_end) {
+    S.sc.done = 1;
+    S.sc.min_dti_bits = 0x7ff0000000000000ULL;
+    S.sc.cfmax_bits = 0ULL;
+  } else {
+    finalize_dt(&S.sc);
+  }
 }
 
 // shared-memory opt-in of a batched stage kernel, done once (before any
@@ -633,8 +688,38 @@ static cudaError_t launch_batch_stage_tl(SimDesc* sims, const int2* items, int n
   return launch_batch_stage_t<false, false, TL>(sims, items, nitems, stage, rk, grid, queue, st);
 }
 
+template <bool MAG, bool GLM, class TL>
+static cudaError_t launch_batch_few_t(SimDesc* sims, const int2* items, int nitems, int stage, int rk,
+                                      cudaStream_t st) {
+  static bool attr = false;
+  if (!attr) {  // rebuilding a batch's work list comes here with no items, outside any capture
+    const cudaError_t e = cudaFuncSetAttribute(batch_few_kernel<MAG, GLM, TL>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)sizeof(SmemT<TL, MAG>));
+    if (e != cudaSuccess) return e;
+    attr = true;
+  }
+  if (nitems == 0) return cudaSuccess;
+  batch_few_kernel<MAG, GLM, TL><<<nitems, TL::NT, sizeof(SmemT<TL, MAG>), st>>>(sims, items, stage, rk);
+  return cudaGetLastError();
+}
+
+template <class TL>
+static cudaError_t launch_batch_few_tl(SimDesc* sims, const int2* items, int nitems, bool mag, bool glm, int stage,
+                                       int rk, cudaStream_t st) {
+  constexpr bool multi = TL::TY > 1;  // GLM exactly on MHD grids of 2 or 3 dimensions
+  if (!mag) return launch_batch_few_t<false, false, TL>(sims, items, nitems, stage, rk, st);
+  if (glm != multi) return cudaErrorInvalidValue;
+  return launch_batch_few_t<true, multi, TL>(sims, items, nitems, stage, rk, st);
+}
+
 cudaError_t launch_batch_stage(SimDesc* sims, const int2* items, int nitems, int tid, bool mag, bool glm, int stage,
                                int rk, int precision, int grid, int* queue, cudaStream_t st) {
+  switch (tid) {
+    case 5: return launch_batch_few_tl<F3D>(sims, items, nitems, mag, glm, stage, rk, st);
+    case 6: return launch_batch_few_tl<F2D>(sims, items, nitems, mag, glm, stage, rk, st);
+    case 7: return launch_batch_few_tl<F1D>(sims, items, nitems, mag, glm, stage, rk, st);
+  }
   if (precision == 1)
     return launch_batch_stage_mixed(sims, items, nitems, tid, mag, glm, stage, rk, grid, queue, st);
   switch (tid) {
@@ -675,21 +760,25 @@ int batch_stage_blocks_per_sm(int tid, bool mag, bool glm, int precision) {
 }
 
 template <class TL>
-static void batch_cfl_tl(SimDesc* sims, const int2* items, int nitems, bool mag, int grid, cudaStream_t st) {
+static void batch_cfl_tl(SimDesc* sims, const int2* items, int nitems, bool mag, int after, int grid,
+                         cudaStream_t st) {
   if (mag)
-    batch_cfl_kernel<true, TL><<<grid, TL::NT, 0, st>>>(sims, items, nitems);
+    batch_cfl_kernel<true, TL><<<grid, TL::NT, 0, st>>>(sims, items, nitems, after);
   else
-    batch_cfl_kernel<false, TL><<<grid, TL::NT, 0, st>>>(sims, items, nitems);
+    batch_cfl_kernel<false, TL><<<grid, TL::NT, 0, st>>>(sims, items, nitems, after);
 }
 
-cudaError_t launch_batch_cfl(SimDesc* sims, const int2* items, int nitems, int tid, bool mag, int grid,
+cudaError_t launch_batch_cfl(SimDesc* sims, const int2* items, int nitems, int tid, bool mag, int after, int grid,
                              cudaStream_t st) {
   switch (tid) {
-    case 0: batch_cfl_tl<T3D>(sims, items, nitems, mag, grid, st); break;
-    case 1: batch_cfl_tl<T3D4>(sims, items, nitems, mag, grid, st); break;
-    case 2: batch_cfl_tl<T2D>(sims, items, nitems, mag, grid, st); break;
-    case 3: batch_cfl_tl<T2D8>(sims, items, nitems, mag, grid, st); break;
-    default: batch_cfl_tl<T1D>(sims, items, nitems, mag, grid, st); break;
+    case 0: batch_cfl_tl<T3D>(sims, items, nitems, mag, after, grid, st); break;
+    case 1: batch_cfl_tl<T3D4>(sims, items, nitems, mag, after, grid, st); break;
+    case 2: batch_cfl_tl<T2D>(sims, items, nitems, mag, after, grid, st); break;
+    case 3: batch_cfl_tl<T2D8>(sims, items, nitems, mag, after, grid, st); break;
+    case 5: batch_cfl_tl<F3D>(sims, items, nitems, mag, after, grid, st); break;
+    case 6: batch_cfl_tl<F2D>(sims, items, nitems, mag, after, grid, st); break;
+    case 7: batch_cfl_tl<F1D>(sims, items, nitems, mag, after, grid, st); break;
+    default: batch_cfl_tl<T1D>(sims, items, nitems, mag, after, grid, st); break;
   }
   return cudaGetLastError();
 }
