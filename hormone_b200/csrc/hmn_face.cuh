@@ -167,8 +167,8 @@ __device__ __forceinline__ bool face_flux_with(PL pl, PR pr, SL sl, SR sr, doubl
     b3l = pl(Q_B + c2) + dx1 * sl(S_B + c2);
     b3r = pr(Q_B + c2) - dx2 * sr(S_B + c2);
     // phi is never reconstructed: its slope is identically zero (allocations.f90)
-    phil = pl(Q_PHI) + dx1 * 0.0;
-    phir = pr(Q_PHI) - dx2 * 0.0;
+    phil = pl(Q_PHI);
+    phir = pr(Q_PHI);
   }
   const double eil = get_eint<MAG>(el, dl, v1l, v2l, v3l, b1l, b2l, b3l);
   const double eir = get_eint<MAG>(er, dr, v1r, v2r, v3r, b1r, b2r, b3r);

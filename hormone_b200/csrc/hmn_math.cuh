@@ -44,29 +44,31 @@ struct PlainDiv {
   __device__ __forceinline__ T root(T x) { return sqrt(x); }
 };
 
+// x with its sign flipped where s is negative: sign(1, s) * x, exactly.
+__device__ __forceinline__ double flip(double x, double s) {
+  return __hiloint2double(__double2hiint(x) ^ (__double2hiint(s) & (int)0x80000000), __double2loint(x));
+}
+
 // Generalised minmod with theta = 1.4 on inverse spacings (fluxlimiter.f90:40-56).
-// i0 = 1/dx(c), i1 = 1/dx(c+1), isum = i0 + i1; risum = dv.rec(isum).
+// i0 = 1/dx(c), i1 = 1/dx(c+1), isum = i0 + i1; risum = dv.rec(isum).  The
+// reference multiplies by sign(1, x); that product is a flip of the sign bit,
+// and a factor taken as |x| costs nothing, so four FP64 multiplications per
+// variable become three logic operations (here as in lim_mmc, where the
+// quotient's numerator takes its sign by copysign).
 template <class D>
 __device__ __forceinline__ double lim_minmod(double u0, double u1, double u2, double i0, double i1, double isum,
                                              D& dv, double risum) {
-  double x = 1.4 * (u2 - u1) * i1;
-  double y = 1.4 * (u1 - u0) * i0;
-  double z = dv.div((u2 - u0) * i0 * i1, isum, risum);
-  double s = fsign(1.0, x);
+  const double x = 1.4 * (u2 - u1) * i1;
+  const double y = 1.4 * (u1 - u0) * i0;
+  const double z = dv.div((u2 - u0) * i0 * i1, isum, risum);
   double m = fabs(x);
-  m = fmin2(m, s * y);
-  m = fmin2(m, s * z);
-  return s * fmax2(0.0, m);
+  m = fmin2(m, flip(y, x));
+  m = fmin2(m, flip(z, x));
+  return copysign(fmax2(0.0, m), x);
 }
 __device__ __forceinline__ double lim_minmod(double u0, double u1, double u2, double i0, double i1, double isum) {
-  double x = 1.4 * (u2 - u1) * i1;
-  double y = 1.4 * (u1 - u0) * i0;
-  double z = (u2 - u0) * i0 * i1 / isum;
-  double s = fsign(1.0, x);
-  double m = fabs(x);
-  m = fmin2(m, s * y);
-  m = fmin2(m, s * z);
-  return s * fmax2(0.0, m);
+  PlainDiv dv;
+  return lim_minmod(u0, u1, u2, i0, i1, isum, dv, isum);
 }
 
 // Modified MC (fluxlimiter.f90:58-75).  Grid factors precomputed per cell:
@@ -76,23 +78,17 @@ __device__ __forceinline__ double lim_minmod(double u0, double u1, double u2, do
 template <class D>
 __device__ __forceinline__ double lim_mmc(double u0, double u1, double u2, double cf, double cb, double ga, double gb,
                                           D& dv, double rga, double rgb) {
-  double top = dv.div((u1 - u0) * ga, gb, rgb);
-  double bot = u2 - u1;
-  double sig = fsign(1.0, bot);
-  double m = sig * 0.5 * (bot + top);
-  m = fmin2(m, sig * cf * bot);
-  m = fmin2(m, sig * cb * top);
-  return dv.div(sig * fmax2(0.0, m), ga, rga);
+  const double bot = u2 - u1, a = fabs(bot);
+  const double t = flip(dv.div((u1 - u0) * ga, gb, rgb), bot);
+  double m = 0.5 * (a + t);
+  m = fmin2(m, cf * a);
+  m = fmin2(m, cb * t);
+  return dv.div(copysign(fmax2(0.0, m), bot), ga, rga);
 }
 __device__ __forceinline__ double lim_mmc(double u0, double u1, double u2, double cf, double cb, double ga,
                                           double gb) {
-  double top = (u1 - u0) * ga / gb;
-  double bot = u2 - u1;
-  double sig = fsign(1.0, bot);
-  double m = sig * 0.5 * (bot + top);
-  m = fmin2(m, sig * cf * bot);
-  m = fmin2(m, sig * cb * top);
-  return sig * fmax2(0.0, m) / ga;
+  PlainDiv dv;
+  return lim_mmc(u0, u1, u2, cf, cb, ga, gb, dv, ga, gb);
 }
 
 // Internal energy from total energy (eos.f90:846-866).
@@ -192,18 +188,36 @@ __device__ __forceinline__ void hlld(T f[9], T cfl, T cfr, T v1l, T v1r, T v2l, 
   const T vbaa = v2aa * b2aa + v3aa * b3aa;
   const T eraa = era + s1 * sqra * ((v2ra * b2ra + v3ra * b3ra) - vbaa);
   const T elaa = ela - s1 * sqla * ((v2la * b2la + v3la * b3la) - vbaa);
-  // branch-free selection of the state at x/t = 0 (hlldflux.f90:113-145)
-  const T signsm = fsign(h, sm);
-  const T wsla = h + fsign(h, sla);
-  const T wsra = h + fsign(h, -sra);
-  const T wslr = h - fsign(h, sla * sra);
-  const T d = (h + signsm) * dla0 + (h - signsm) * dra0;
-  const T v2 = wsla * v2la + wslr * v2aa + wsra * v2ra;
-  const T v3 = wsla * v3la + wslr * v3aa + wsra * v3ra;
-  const T bb2 = wsla * b2la + wslr * b2aa + wsra * b2ra;
-  const T bb3 = wsla * b3la + wslr * b3aa + wsra * b3ra;
-  const T e = wsla * ela + (h - fsign(h, sla * sm)) * elaa + (h + fsign(h, -(sm * sra))) * eraa +
-                   (h - fsign(h, sra)) * era;
+  T d, v2, v3, bb2, bb3, e;
+  if constexpr (D::flags) {
+    // The reference adds each state times 0 or 1, by the signs of sm, sla <= sm
+    // and sra >= sm.  A finite state times 0 adds nothing, so the state can be
+    // picked: 24 selects instead of 42 FP64 operations.  All are finite unless
+    // refused: the quotients by their operands, the energies here.  (Where a
+    // zero's sign picks otherwise there, every flux has a zero factor.)
+    dvp.template need_below<1000>(elaa);
+    dvp.template need_below<1000>(eraa);
+    const bool ml = !(sm < zero), la = !(sla < zero), ra = sra < zero;
+    d = ml ? dla0 : dra0;
+    v2 = la ? v2la : (ra ? v2ra : v2aa);
+    v3 = la ? v3la : (ra ? v3ra : v3aa);
+    bb2 = la ? b2la : (ra ? b2ra : b2aa);
+    bb3 = la ? b3la : (ra ? b3ra : b3aa);
+    e = la ? ela : (ra ? era : (ml ? elaa : eraa));
+  } else {
+    // branch-free selection of the state at x/t = 0 (hlldflux.f90:113-145)
+    const T signsm = fsign(h, sm);
+    const T wsla = h + fsign(h, sla);
+    const T wsra = h + fsign(h, -sra);
+    const T wslr = h - fsign(h, sla * sra);
+    d = (h + signsm) * dla0 + (h - signsm) * dra0;
+    v2 = wsla * v2la + wslr * v2aa + wsra * v2ra;
+    v3 = wsla * v3la + wslr * v3aa + wsra * v3ra;
+    bb2 = wsla * b2la + wslr * b2aa + wsra * b2ra;
+    bb3 = wsla * b3la + wslr * b3aa + wsra * b3ra;
+    e = wsla * ela + (h - fsign(h, sla * sm)) * elaa + (h + fsign(h, -(sm * sra))) * eraa +
+                     (h - fsign(h, sra)) * era;
+  }
   const T v1 = sm, p = pta;
   const T dv = d * v1;
   f[0] = dv;
