@@ -807,15 +807,12 @@ static int fetch_scalars(hmn_ctx* ctx) {
   return HMN_OK;
 }
 
+// The device clock of a host-driven step, set by a launch on the step's stream:
+// its arguments travel with it, where a copy from the stack and a memset made
+// the host wait for the stream before every step.
 static int push_times(hmn_ctx* ctx, double time, double t_out, double t_end) {
-  // only the three time fields change; write them individually
-  double tv[3] = {time, t_out, t_end};
-  static_assert(offsetof(DevScalars, t_out) == offsetof(DevScalars, time) + sizeof(double), "layout");
-  static_assert(offsetof(DevScalars, t_end) == offsetof(DevScalars, time) + 2 * sizeof(double), "layout");
-  double* dst = &ctx->sc->time;
-  CK(cudaMemcpyAsync(dst, tv, sizeof(tv), cudaMemcpyHostToDevice, ctx->st), "times");
-  CK(cudaMemsetAsync(&ctx->sc->done, 0, sizeof(int), ctx->st), "times");
-  CK(cudaStreamSynchronize(ctx->st), "sync");
+  CK(launch_set_times(ctx->sc, time, t_out, t_end, ctx->st), "times");
+  ctx->launches += 1;
   return HMN_OK;
 }
 
@@ -1129,6 +1126,7 @@ extern "C" int hmn_cfl_local(hmn_ctx* ctx, double time, double t_out, double t_e
   if (!ctx) return HMN_EINVAL;
   int rc = push_times(ctx, time, t_out, t_end);
   if (rc) return rc;
+  CK(cudaStreamSynchronize(ctx->st), "sync");  // slabs: the stages before are finished here
   CK(launch_cfl_cells(ctx->G, ctx->pbuf[ctx->pcur], ctx->plane, ctx->par.gamma, ctx->sc, ctx->mag,
                       blocks_for(ctx), ctx->st),
      "cfl");

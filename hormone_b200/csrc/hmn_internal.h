@@ -207,6 +207,7 @@ bool march_enabled();
 void march_chunks(const int n[3], int* lz, int* ntx, int* nty, int* nch);
 // up to R.nsteps steps of a small grid in one cooperative launch of at most
 // one CTA per tile (hmn_small.cu); *grid receives the CTA count
+int sm_count();  // of the current device (asked once)
 int small_run_tile(const int tile[3], const int n[3], int nsm, bool sph, int out[3]);
 cudaError_t launch_small_run(const GridDev& G, const SmallRun& R, bool mag, bool glm, bool sph, const int tile[3],
                              cudaStream_t st, int* grid);
@@ -222,6 +223,8 @@ cudaError_t launch_pack_zhalos(const double* P, const int n[3], int nplanes, dou
                                int nblocks, cudaStream_t st);
 cudaError_t launch_cfl(const GridDev& G, const double* P, size_t plane, double gamma, DevScalars* sc, bool mag,
                        int nblocks, cudaStream_t st);
+// the device clock at the start of a host-driven step: the three times, done = 0
+cudaError_t launch_set_times(DevScalars* sc, double time, double t_out, double t_end, cudaStream_t st);
 cudaError_t launch_prim_init(double* P, size_t plane, bool mag, int nblocks, cudaStream_t st);
 cudaError_t launch_prim_from_u(const double* U, double* P, size_t plane, bool mag, bool glm, int nblocks,
                                cudaStream_t st);

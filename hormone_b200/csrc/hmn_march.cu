@@ -457,6 +457,8 @@ cudaError_t launch_mag(const GridDev& G, const StageArgs& A, bool mag, bool glm,
   return launch_lim<false, false, PUSH>(G, A, LZ, ntx, nty, nch, st);
 }
 
+}  // namespace
+
 int sm_count() {
   static int n = 0;
   if (n == 0) {
@@ -467,8 +469,6 @@ int sm_count() {
   }
   return n;
 }
-
-}  // namespace
 
 // HMN_MARCH=0 keeps 3-D Cartesian grids on the tile kernel (read at every
 // launch; a captured CUDA graph keeps the kernel it was captured with)

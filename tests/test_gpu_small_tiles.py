@@ -9,6 +9,7 @@ from hormone_b200 import config, grid as G, ic
 from hormone_b200.sim import Simulation
 
 import cases
+from test_gpu_parity import run_pair
 
 pytestmark = pytest.mark.gpu
 
@@ -62,3 +63,19 @@ def test_spherical_tiles(monkeypatch, n):
     monkeypatch.setenv("HMN_SMALL", "0")
     v, t0 = _run(cfg, prims, 3)
     assert t == t0 and np.array_equal(u, v)
+
+
+# steps driven call by call take the small tiles of 1-D and 2-D grids too
+# (launch_stage_few, hmn_kernels.cu): against the oracle
+@pytest.mark.parametrize("n", [(30, 1, 1), (31, 1, 1), (4440, 1, 1), (4441, 1, 1), (8, 8, 1), (9, 7, 1), (96, 96, 1),
+                               (97, 97, 1), (256, 149, 1)])
+@pytest.mark.parametrize("mag", [False, True])
+def test_host_driven_steps(n, mag):
+    cfg, prims = _case(n, mag)
+    run_pair(cfg, prims, 2)
+
+
+@pytest.mark.parametrize("n", [(31, 1, 1), (17, 16, 1), (128, 80, 1)])
+def test_host_driven_spherical_steps(n):
+    cfg, prims = cases.spherical(n=n, mag=n[1] > 1)
+    run_pair(cfg, prims, 2)
