@@ -105,6 +105,7 @@ struct DevScalars {
   int err_code, err_i, err_j, err_k;
   int done;  // set by advance_kernel once time >= t_end; later launches of hmn_run skip their work
   int tn;
+  int cfl_bad;  // batches: 1 + tn of the first state whose CFL reduction met a bad cell
 };
 
 // Arguments of one fused RK stage launch (hmn_kernels.cu: stage_kernel).

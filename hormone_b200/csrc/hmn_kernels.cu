@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(TL::NT, TL::MINB) batch_few_kernel(SimDesc* si
     return;
   }
   double my_dti = __longlong_as_double(0x7ff0000000000000LL), my_cf = 0.0;
-  stage_tile_exact<MAG, GLM, TL, false, false, true>(S.G, A, sm, w.y, nullptr, &my_dti, &my_cf);
+  stage_tile_exact<MAG, GLM, TL, false, false, true>(S.G, A, sm, w.y, nullptr, &my_dti, &my_cf, 1);
   cfl_block_reduce(my_dti, my_cf, &S.sc);
 }
 
@@ -653,7 +653,7 @@ __global__ void __launch_bounds__(TL::NT) batch_cfl_kernel(SimDesc* sims, const 
       if (cx >= T[0] || cy >= T[1] || cz >= T[2]) continue;
       const int i = t0[0] + cx, j = t0[1] + cy, k = t0[2] + cz;
       double dti, cfm;
-      if (!cfl_cell<MAG>(G, P, S.plane, S.gamma, cidx(G, i, j, k), i, j, k, &S.sc, dti, cfm)) continue;
+      if (!cfl_cell<MAG>(G, P, S.plane, S.gamma, cidx(G, i, j, k), i, j, k, &S.sc, dti, cfm, after > 0)) continue;
       my_cf = fmax2(my_cf, cfm);
       my_dti = fmin2(my_dti, dti);
     }
@@ -677,6 +677,7 @@ __global__ void batch_advance_kernel(SimDesc* sims, int nsims) {
   if (!S.active || S.sc.done || S.held) return;
   S.sc.time = S.sc.time + S.sc.dt;
   S.sc.tn = S.sc.tn + 1;
+  next_step_error(&S.sc);
   S.pcur = (S.pcur + S.rktype) & 1;
   if (S.rktype == 1) {
     double* t = S.U[0];

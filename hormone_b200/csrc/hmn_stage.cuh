@@ -173,13 +173,15 @@ __device__ __forceinline__ void axis_pass(const GridDev& G, const StageArgs& A, 
 template <bool MAG>
 __device__ __forceinline__ bool cfl_values(const GridDev& G, double gamma, double d, double eint, double v1, double v2,
                                            double v3, double b1, double b2, double b3, int i, int j, int k,
-                                           DevScalars* sc, double& dti, double& cfm);
+                                           DevScalars* sc, double& dti, double& cfm, int ahead = -1);
 
 // CFLOUT: also fold dti and the signal speed of each new cell (dti_cell,
-// the next step's CFL reduction) into *cdti (min) and *ccf (max).
+// the next step's CFL reduction) into *cdti (min) and *ccf (max); ahead as
+// cfl_values.
 template <bool MAG, bool GLM, class TL, bool SPH = false, bool PUSH = false, bool CFLOUT = false>
 __device__ __forceinline__ void stage_tile_exact(const GridDev& G, const StageArgs& A, SmemT<TL, MAG>& sm, int tile_id,
-                                                 const TmaMaps* tm, double* cdti = nullptr, double* ccf = nullptr) {
+                                                 const TmaMaps* tm, double* cdti = nullptr, double* ccf = nullptr,
+                                                 int ahead = -1) {
   const int tid = threadIdx.x;
 
   int bid = tile_id;
@@ -303,7 +305,7 @@ __device__ __forceinline__ void stage_tile_exact(const GridDev& G, const StageAr
   if (eint <= 0.0) record_error(A.sc, kENEG_EINT, i, j, k);
   if constexpr (CFLOUT) {
     double dti, cfm;
-    if (cfl_values<MAG>(G, A.gamma, d, eint, v1, v2, v3, b1, b2, b3, i, j, k, A.sc, dti, cfm)) {
+    if (cfl_values<MAG>(G, A.gamma, d, eint, v1, v2, v3, b1, b2, b3, i, j, k, A.sc, dti, cfm, ahead)) {
       *ccf = fmax2(*ccf, cfm);
       *cdti = fmin2(*cdti, dti);
     }
@@ -332,16 +334,34 @@ __device__ __forceinline__ void stage_tile_exact(const GridDev& G, const StageAr
 
 __device__ __forceinline__ unsigned long long dbits(double x) { return (unsigned long long)__double_as_longlong(x); }
 
+// A batch reduces the CFL quantities of a state at the end of the step that made
+// it, where the reference does so at the start of the next one.  A bad cell
+// is an error of that next step, which a finished simulation never takes: it
+// is kept here (ahead: 0 for the current state, 1 for the one the running step
+// makes) and becomes the simulation's error when the step from that state has
+// run (next_step_error).
+__device__ __forceinline__ void kept_for_next_step(DevScalars* sc, int ahead) {
+  atomicCAS(&sc->cfl_bad, 0, sc->tn + ahead + 1);
+}
+// after the clock's advance: tn - 1 is the state that the step started from
+__device__ __forceinline__ void next_step_error(DevScalars* sc) {
+  if (sc->cfl_bad != 0 && sc->tn >= sc->cfl_bad) record_error(sc, kENEG_EINT, -1, -1, -1);
+}
+
 // dti and the largest signal speed of one cell (dti_cell, timestep.f90:125-183,
-// eostype 0); false (and the error recorded) if eint <= 0 or d <= 0
+// eostype 0); false if eint <= 0 or d <= 0, with the error recorded (ahead < 0)
+// or kept for the next step
 template <bool MAG>
 __device__ __forceinline__ bool cfl_values(const GridDev& G, double gamma, double d, double eint, double v1, double v2,
                                            double v3, double b1, double b2, double b3, int i, int j, int k,
-                                           DevScalars* sc, double& dti, double& cfm) {
+                                           DevScalars* sc, double& dti, double& cfm, int ahead) {
   const double gm1 = gamma - 1.0;
   const double off0 = G.solve[0] ? 1.0 : 0.0, off1 = G.solve[1] ? 1.0 : 0.0, off2 = G.solve[2] ? 1.0 : 0.0;
   if (eint <= 0.0 || d <= 0.0) {
-    record_error(sc, kENEG_EINT, i, j, k);
+    if (ahead < 0)
+      record_error(sc, kENEG_EINT, i, j, k);
+    else
+      kept_for_next_step(sc, ahead);
     return false;
   }
   const double p = gm1 * eint;
@@ -384,7 +404,8 @@ __device__ __forceinline__ bool cfl_values(const GridDev& G, double gamma, doubl
 // the same for cell c of the primitive planes P
 template <bool MAG>
 __device__ __forceinline__ bool cfl_cell(const GridDev& G, const double* P, size_t plane, double gamma, size_t c,
-                                         int i, int j, int k, DevScalars* sc, double& dti, double& cfm) {
+                                         int i, int j, int k, DevScalars* sc, double& dti, double& cfm,
+                                         int ahead = -1) {
   const double d = P[c], eint = P[PEINT * plane + c];
   const double v1 = P[plane + c], v2 = P[2 * plane + c], v3 = P[3 * plane + c];
   double b1 = 0.0, b2 = 0.0, b3 = 0.0;
@@ -393,7 +414,7 @@ __device__ __forceinline__ bool cfl_cell(const GridDev& G, const double* P, size
     b2 = P[6 * plane + c];
     b3 = P[7 * plane + c];
   }
-  return cfl_values<MAG>(G, gamma, d, eint, v1, v2, v3, b1, b2, b3, i, j, k, sc, dti, cfm);
+  return cfl_values<MAG>(G, gamma, d, eint, v1, v2, v3, b1, b2, b3, i, j, k, sc, dti, cfm, ahead);
 }
 
 // block-wide min(dti), max(cf) folded into the simulation's reduction slots
