@@ -514,8 +514,10 @@ static int rebuild(hmn_batch* b) {
     if (!b->side[c]) BCK(cudaStreamCreateWithFlags(&b->side[c], cudaStreamNonBlocking), "side stream");
     if (!b->join[c]) BCK(cudaEventCreateWithFlags(&b->join[c], cudaEventDisableTiming), "join event");
   }
-  b->dirty = false;
-  return start_steps(b);
+  // the list stands once its steps can start; until then the next step makes it anew
+  const int rc = start_steps(b);
+  b->dirty = rc != HMN_OK;
+  return rc;
 }
 
 // Run f(class, stream) for every class: the first on the batch's stream, the
