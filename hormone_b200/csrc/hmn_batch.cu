@@ -43,6 +43,7 @@ struct Klass {
   int grid;          // persistent CTAs of the stage launches
   bool dynamic;      // stage launches take items from the shared counter
   int* queue;        // that counter: {next item, CTAs finished}
+  bool fresh;        // holds simulations that have not stepped yet
 };
 
 // Steps captured in one graph: between two replays the GPU idles a few
@@ -341,6 +342,7 @@ extern "C" int hmn_batch_add(hmn_batch* b, const hmn_grid* grid, const hmn_param
   S.rktype = par->rktype;
   S.glm = glm;
   S.active = 1;
+  S.fresh = 1;
   S.gamma = par->gamma;
   S.gm1 = par->gamma - 1.0;
   S.damp = std::exp(-par->alpha9wave * par->courant);
@@ -437,7 +439,7 @@ static int rebuild(hmn_batch* b) {
     for (int m = 0; m < 3; m++) {
       const bool mag = m > 0, glm = m == 2;
       const int sweep = b->sweep[kind];
-      Klass k{kind, b->tile_id[kind], false, mag, glm, (int)items.size(), 0, 0, sweep == HMN_SWEEP_DYNAMIC, nullptr};
+      Klass k{kind, b->tile_id[kind], false, mag, glm, (int)items.size(), 0, 0, sweep == HMN_SWEEP_DYNAMIC, nullptr, false};
       std::vector<int> sims;
       int most_tiles = 0;
       for (int s = 0; s < b->max_sims; s++) {
@@ -446,6 +448,7 @@ static int rebuild(hmn_batch* b) {
             b->h_sims[s].held)
           continue;
         sims.push_back(s);
+        k.fresh |= b->h_sims[s].fresh != 0;
         most_tiles = std::max(most_tiles, si.ntiles);
       }
       // items of each listed simulation: the schedule's tiles, or smaller ones
@@ -544,17 +547,20 @@ static int enqueue_cfl(hmn_batch* b, const Klass& k, int after, cudaStream_t st)
   return HMN_OK;
 }
 
-// dt of the listed simulations' current states; every step then ends with the
-// next one's.  (For a simulation that has stepped before it is the dt that its
-// last step left, formed again from the same state.)
+// The first dt of the simulations that have not stepped yet; every step then
+// ends with the next one's, which a simulation keeps while others join, leave
+// or are held.
 static int start_steps(hmn_batch* b) {
-  if (b->classes.empty()) return HMN_OK;
+  int started = 0;
   for (const Klass& k : b->classes) {
+    if (!k.fresh) continue;
     const int rc = enqueue_cfl(b, k, 0, b->st);
     if (rc) return rc;
+    started++;
   }
+  if (started == 0) return HMN_OK;
   BCK(launch_batch_finalize(b->d_sims, b->max_sims, b->st), "batch finalize");
-  b->launches += (long long)b->classes.size() + 1;
+  b->launches += started + 1;
   return HMN_OK;
 }
 

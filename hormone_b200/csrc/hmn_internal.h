@@ -184,6 +184,7 @@ struct SimDesc {
   int nvar, limiter, rktype, glm;
   int active;         // 0 for a free slot
   int held;           // 1: left out of the steps until released (hmn_batch_set_held)
+  int fresh;          // 1: added, and the dt of its first step not yet formed
   double gamma, gm1;
   double damp;        // phidamp factor exp(-alpha9wave*courant)
   double phifac;      // pending phidamp factor for the next stage 1

@@ -629,13 +629,14 @@ __global__ void __launch_bounds__(TL::NT, (MAG ? TL::MINB : TL::MINBH)) batch_st
 }
 
 // CFL quantities of the state `after` RK stages past the current one (0: the
-// current state; rk: the state the step's last stage wrote)
+// current state, of the fresh simulations; rk: the state the step's last stage
+// wrote)
 template <bool MAG, class TL>
 __global__ void __launch_bounds__(TL::NT) batch_cfl_kernel(SimDesc* sims, const int2* items, int nitems, int after) {
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const int2 w = items[it];
     SimDesc& S = sims[w.x];
-    if (!S.active || S.sc.done) continue;
+    if (!S.active || S.sc.done || (after == 0 && !S.fresh)) continue;
     const GridDev& G = S.G;
     int bid = w.y, t0[3], T[3];
     constexpr int TT[3] = {TL::TX, TL::TY, TL::TZ};
@@ -663,8 +664,9 @@ __global__ void __launch_bounds__(TL::NT) batch_cfl_kernel(SimDesc* sims, const 
 
 __global__ void batch_finalize_kernel(SimDesc* sims, int nsims) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsims || !sims[s].active || sims[s].sc.done || sims[s].held) return;
+  if (s >= nsims || !sims[s].active || sims[s].sc.done || sims[s].held || !sims[s].fresh) return;
   finalize_dt(&sims[s].sc);
+  sims[s].fresh = 0;
 }
 
 // time += dt, tn += 1, end check (hormone.f90:147-155); primitive buffer

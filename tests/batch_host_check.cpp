@@ -97,8 +97,9 @@ cudaError_t launch_prim_init(double*, size_t, bool, int, cudaStream_t) { return 
 cudaError_t launch_prim_from_u(const double*, double*, size_t, bool, bool, int, cudaStream_t) { return cudaSuccess; }
 
 constexpr double kDt = 0.25;
-static void reduce(SimDesc* sims, const int2* items, int n) {
+static void reduce(SimDesc* sims, const int2* items, int n, bool fresh) {
   for (int i = 0; i < n; i++) {
+    if (fresh && !sims[items[i].x].fresh) continue;
     const double dti = kDt;
     memcpy(&sims[items[i].x].sc.min_dti_bits, &dti, sizeof(dti));
   }
@@ -108,19 +109,19 @@ static void next_dt(SimDesc& S) {
   S.sc.min_dti_bits = 0x7ff0000000000000ULL;
 }
 cudaError_t launch_batch_cfl(SimDesc* sims, const int2* items, int n, int, bool, int after, int, cudaStream_t) {
-  return launch(after ? "cfl" : "cfl0", [=] { reduce(sims, items, n); });
+  return launch(after ? "cfl" : "cfl0", [=] { reduce(sims, items, n, after == 0); });
 }
 cudaError_t launch_batch_finalize(SimDesc* sims, int n, cudaStream_t) {
   return launch("finalize", [=] {
     for (int s = 0; s < n; s++)
-      if (sims[s].active && !sims[s].sc.done && !sims[s].held) next_dt(sims[s]);
+      if (sims[s].active && !sims[s].sc.done && !sims[s].held && sims[s].fresh) next_dt(sims[s]), sims[s].fresh = 0;
   });
 }
 cudaError_t launch_batch_stage(SimDesc* sims, const int2* items, int n, int tile, bool, bool, int stage, int rk, int, int,
                                int*, cudaStream_t) {
   if (n == 0) return cudaSuccess;
   return launch(tile >= 5 ? "few" : "stage", [=] {
-    if (tile >= 5 && stage == rk) reduce(sims, items, n);
+    if (tile >= 5 && stage == rk) reduce(sims, items, n, false);
   });
 }
 cudaError_t launch_batch_advance(SimDesc* sims, int n, cudaStream_t) {
@@ -185,4 +186,27 @@ static int check_failed_start() {
   return 0;
 }
 
-int main() { return check_failed_start(); }
+// the reduction that starts a simulation runs once for it, and not for those
+// that others join, leave or pass by
+static int check_start_once() {
+  hmn_batch* b = nullptr;
+  CHECK(hmn_batch_create(1 << 26, 8, 0, 3, &b) == HMN_OK);
+  trace.clear();
+  const int s0 = add(b, 400, 300, true), s1 = add(b, 30, 1, true);  // one class of many items, one of few
+  CHECK(hmn_batch_step(b, 2) == HMN_OK && ran("cfl0") == 2 && ran("finalize") == 1);
+  int held[8] = {};
+  held[s1] = 1;
+  CHECK(hmn_batch_set_held(b, held) == HMN_OK && hmn_batch_step(b, 3) == HMN_OK);
+  held[s1] = 0;
+  CHECK(hmn_batch_set_held(b, held) == HMN_OK && hmn_batch_step(b, 1) == HMN_OK);
+  CHECK(ran("cfl0") == 2 && ran("finalize") == 1);
+  const int s2 = add(b, 60, 1, true);  // the class of few items starts its new simulation only
+  CHECK(hmn_batch_step(b, 4) == HMN_OK && ran("cfl0") == 3 && ran("finalize") == 2);
+  CHECK(at(b, s0, 10) && at(b, s1, 7) && at(b, s2, 4));
+  CHECK(hmn_batch_remove(b, s0) == HMN_OK && hmn_batch_step(b, 1) == HMN_OK && ran("cfl0") == 3);
+  CHECK(at(b, s1, 8) && at(b, s2, 5));
+  hmn_batch_destroy(b);
+  return 0;
+}
+
+int main() { return check_failed_start() || check_start_once(); }
