@@ -209,4 +209,34 @@ static int check_start_once() {
   return 0;
 }
 
-int main() { return check_failed_start() || check_start_once(); }
+// the same steps whether they are launched directly or replayed from graphs,
+// and graphs only for a list that lasts
+static int check_graphs() {
+  hmn_batch* b = nullptr;
+  CHECK(hmn_batch_create(1 << 26, 8, 0, 3, &b) == HMN_OK);
+  const int s0 = add(b, 400, 300, true), s1 = add(b, 30, 1, true);
+  captures = 0;
+  trace.clear();
+  int steps = 0;
+  const auto step = [&](int n) {
+    steps += n;
+    return hmn_batch_step(b, n) == HMN_OK && ran("advance") == steps && ran("few") == 3 * steps &&
+           ran("cfl") == steps;
+  };
+  CHECK(step(kGraphAfter - 1) && step(1) && captures == 0);
+  CHECK(step(1) && captures == 1);
+  CHECK(step(kManyAfter - kGraphAfter - 1) && captures == 1);
+  CHECK(step(kManySteps - 1) && step(1) && captures == 1);
+  CHECK(step(3 * kManySteps + 2) && captures == 2);
+  CHECK(step(kManySteps) && step(2) && captures == 2);
+  CHECK(hmn_batch_launch_count(b) == 2 + (long long)trace.size());  // two launches of the additions
+  CHECK(at(b, s0, steps) && at(b, s1, steps));
+  const int s2 = add(b, 20, 1, true);
+  CHECK(step(kGraphAfter) && captures == 2);
+  CHECK(step(kManyAfter + kManySteps - kGraphAfter) && captures == 4);
+  CHECK(at(b, s0, steps) && at(b, s1, steps) && at(b, s2, kManyAfter + kManySteps));
+  hmn_batch_destroy(b);
+  return 0;
+}
+
+int main() { return check_failed_start() || check_start_once() || check_graphs(); }
