@@ -313,31 +313,35 @@ static cudaError_t launch_scalar_tiles(const GridDev& G, const StageArgs& A, boo
   return cudaErrorInvalidValue;
 }
 
-// The stage of a small 1-D (x) or 2-D (x-y) grid on the tiles of the persistent
-// small-grid loop, for steps that the host drives call by call or that run in
-// graphs: the stage is as long as one CTA's chain of phases, which is shortest
-// with one warp (30 cells) or three (8x8) per CTA.  A tube of 1024 cells driven
-// call by call, 4 steps: 384 -> 326 us (together with the clock set by a launch
-// instead of a copy and a wait).
+// The stage of a small 1-D (x) or 2-D (x-y) grid on small tiles, for steps that
+// the host drives call by call or that run in graphs: the stage is as long as one
+// CTA's chain of phases, which is shortest with one warp (30 cells) or three (8x8)
+// per CTA, as long as all CTAs are resident at once: four one-warp CTAs per SM
+// (one per scheduler), two of 8x8 with a field and four without.  A step in graphs
+// on them and on the 256-cell and 16x16 tiles, us: with a field 1000 cells 35.1 and
+// 40.2, 18000 37.9 and 40.1, 37000 (1234 tiles) 41.9 and 41.0; 96^2 43.9 and 66.3,
+// 136^2 (289 tiles) 47.7 and 71.4, 150x140 (342) 79.0 and 73.0; hydro 192^2 (576) 40.8
+// and 46.9, 224^2 (784) 61.5 and 54.3.  A tube of 1024 cells driven call by call, 4
+// steps: 384 -> 326 us (together with the clock set by a launch instead of a copy
+// and a wait).
 static cudaError_t launch_stage_few(const GridDev& G, const StageArgs& A, bool mag, bool glm, cudaStream_t st) {
-  int t[3];
-  const bool sph = G.sph.on != 0;
-  if (A.nspc > 0 || !small_run_tile(A.tile, G.n, sm_count(), sph, t)) return cudaErrorNotSupported;
-  const int id = t[0] == 30 ? 0 : (t[0] == 8 && t[1] == 8 && t[2] == 1 ? 1 : (t[0] == 16 && t[1] == 8 ? 2 : -1));
-  if (id < 0) return cudaErrorNotSupported;
+  const int* t = A.tile;
+  const bool line = t[0] == 256 && t[1] == 1 && t[2] == 1, plane = t[0] == 16 && t[1] == 16 && t[2] == 1;
+  if (A.nspc > 0 || !(line || plane)) return cudaErrorNotSupported;
+  const int cut[3] = {line ? 30 : 8, line ? 1 : 8, 1};
   StageArgs B = A;
+  int count = 1;
   for (int a = 0; a < 3; a++) {
-    B.tile[a] = t[a];
-    B.tiles[a] = (G.n[a] + t[a] - 1) / t[a];
+    B.tile[a] = cut[a];
+    B.tiles[a] = (G.n[a] + cut[a] - 1) / cut[a];
+    count *= B.tiles[a];
   }
-  if (sph) {
-    if (id == 0) return launch_stage_sph_tl<Tile<30, 1, 1, 32, 1>>(G, B, mag, glm, st);
-    if (id == 1) return launch_stage_sph_tl<Tile<8, 8, 1, 96, 1>>(G, B, mag, glm, st);
-    return launch_stage_sph_tl<Tile<16, 8, 1, 160, 1>>(G, B, mag, glm, st);
-  }
-  if (id == 0) return launch_stage_tl<Tile<30, 1, 1, 32, 1>>(G, B, mag, glm, nullptr, st);
-  if (id == 1) return launch_stage_tl<Tile<8, 8, 1, 96, 1>>(G, B, mag, glm, nullptr, st);
-  return launch_stage_tl<Tile<16, 8, 1, 160, 1>>(G, B, mag, glm, nullptr, st);
+  if (count > (line || !mag ? 4 : 2) * sm_count()) return cudaErrorNotSupported;
+  if (G.sph.on)
+    return line ? launch_stage_sph_tl<Tile<30, 1, 1, 32, 1>>(G, B, mag, glm, st)
+                : launch_stage_sph_tl<Tile<8, 8, 1, 96, 1>>(G, B, mag, glm, st);
+  return line ? launch_stage_tl<Tile<30, 1, 1, 32, 1>>(G, B, mag, glm, nullptr, st)
+              : launch_stage_tl<Tile<8, 8, 1, 96, 1>>(G, B, mag, glm, nullptr, st);
 }
 
 cudaError_t launch_stage(const GridDev& G, const StageArgs& A, bool mag, bool glm, const TmaMaps* tm,

@@ -172,13 +172,18 @@ cudaError_t launch_mag(const GridDev& G, const SmallRun& R, bool mag, bool glm, 
 
 // The tiles of the persistent loop, by the grid's solved axes (those of the
 // stage tile).  A step is a chain of phases, each as long as one CTA's slopes,
-// faces and cells take, and that grows with the warps that share an SM.  So
-// the grid is cut into the smallest tiles that still give (about) every SM no
-// more than one CTA of the next size up: 1-D tiles of 30 cells are one warp
-// (32 slope cells), and their barriers cost nothing.  The larger tiles compute
-// fewer halo slopes and faces twice and stay for the larger grids.
-// Against the largest tiles throughout: 128x128 MHD, 64 steps 3.84 -> 3.00 ms;
-// 500 radial cells, 64 steps 1.79 -> 1.65 ms.
+// faces and cells take, and as the rounds of tiles that a CTA walks: the grid is
+// cut into small tiles while all of them are resident at once (us per step, 64
+// steps, with a field unless said):
+//  * 1-D: 126 cells (four warps).  64 cells 26.3 (30-cell tiles 30.4, 256-cell
+//    29.3), 500 29.9 (30.2, 34.1), 500 radial hydro 23.0 (24.8, 25.5), 20000 radial
+//    hydro 25.5 (27.8, 27.2), 65536 53.1 (61.8, 58.5): no size is better served by
+//    another.
+//  * 2-D: 8x8 up to two CTAs per SM, then 16x16.  96^2 41.2 (16x16 55.0), 136^2 (289
+//    tiles of 8x8) 46.2 (59.2), 150x140 (342) 81.8 (58.3), 192^2 73.1 (55.2); hydro
+//    136^2 33.1 (42.9), 150x140 55.0 (41.6).
+//  * 3-D: 8x4x4 up to one CTA per SM, then 8x8x8.  24x24x32 (144 tiles of 8x4x4) 62.7
+//    (8x8x8 114.4), 26^3 (196) 115.4 (113.5), 36^3 165 (113.5).
 static int tiles_of(const int n[3], const int t[3]) {
   int c = 1;
   for (int a = 0; a < 3; a++) c *= (n[a] + t[a] - 1) / t[a];
@@ -186,18 +191,13 @@ static int tiles_of(const int n[3], const int t[3]) {
 }
 
 int small_run_tile(const int tile[3], const int n[3], int nsm, bool sph, int out[3]) {
-  static const int one[3][3] = {{30, 1, 1}, {126, 1, 1}, {256, 1, 1}};
-  static const int two[3][3] = {{8, 8, 1}, {16, 8, 1}, {16, 16, 1}};
-  static const int three[2][3] = {{8, 4, 4}, {8, 8, 8}};
-  const int(*t)[3] = nullptr;
-  int kinds = 3;
+  static const int one[3] = {126, 1, 1}, two[2][3] = {{8, 8, 1}, {16, 16, 1}}, three[2][3] = {{8, 4, 4}, {8, 8, 8}};
+  const int* t = nullptr;
   if (tile[0] == 256 && tile[1] == 1 && tile[2] == 1) t = one;
-  if (tile[0] == 16 && tile[1] == 16 && tile[2] == 1) t = two;
-  if (tile[0] == 8 && tile[1] == 8 && tile[2] == 8 && !sph) t = three, kinds = 2;
+  if (tile[0] == 16 && tile[1] == 16 && tile[2] == 1) t = two[tiles_of(n, two[0]) > 2 * nsm];
+  if (tile[0] == 8 && tile[1] == 8 && tile[2] == 8 && !sph) t = three[tiles_of(n, three[0]) > nsm];
   if (t == nullptr) return 0;
-  int k = 0;
-  while (k + 1 < kinds && tiles_of(n, t[k]) > (k == 0 ? 1 : 2) * nsm) k++;
-  for (int a = 0; a < 3; a++) out[a] = t[k][a];
+  for (int a = 0; a < 3; a++) out[a] = t[a];
   return 1;
 }
 
@@ -205,21 +205,12 @@ cudaError_t launch_small_run(const GridDev& G, const SmallRun& R, bool mag, bool
                              cudaStream_t st, int* grid) {
   const int t = tile[0] * 10000 + tile[1] * 100 + tile[2];
   switch (t) {
-    case 300101:
-      return sph ? launch_mag<Tile<30, 1, 1, 32, 2>, true>(G, R, mag, glm, st, grid)
-                 : launch_mag<Tile<30, 1, 1, 32, 2>, false>(G, R, mag, glm, st, grid);
     case 1260101:
       return sph ? launch_mag<Tile<126, 1, 1, 128, 2>, true>(G, R, mag, glm, st, grid)
                  : launch_mag<Tile<126, 1, 1, 128, 2>, false>(G, R, mag, glm, st, grid);
-    case 2560101:
-      return sph ? launch_mag<Tile<256, 1, 1, 288, 2>, true>(G, R, mag, glm, st, grid)
-                 : launch_mag<Tile<256, 1, 1, 288, 2>, false>(G, R, mag, glm, st, grid);
     case 80801:
       return sph ? launch_mag<Tile<8, 8, 1, 96, 2>, true>(G, R, mag, glm, st, grid)
                  : launch_mag<Tile<8, 8, 1, 96, 2>, false>(G, R, mag, glm, st, grid);
-    case 160801:
-      return sph ? launch_mag<Tile<16, 8, 1, 160, 2>, true>(G, R, mag, glm, st, grid)
-                 : launch_mag<Tile<16, 8, 1, 160, 2>, false>(G, R, mag, glm, st, grid);
     case 161601:
       return sph ? launch_mag<Tile<16, 16, 1, 288, 2>, true>(G, R, mag, glm, st, grid)
                  : launch_mag<Tile<16, 16, 1, 288, 2>, false>(G, R, mag, glm, st, grid);

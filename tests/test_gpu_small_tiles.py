@@ -13,8 +13,8 @@ from test_gpu_parity import run_pair
 
 pytestmark = pytest.mark.gpu
 
-# 1-D: 30 cells up to 148 tiles (4440), 126 up to 296 (37296), then 256
-# 2-D: 8x8 up to 148 tiles, 16x8 up to 296, then 16x16
+# 1-D: 126 cells
+# 2-D: 8x8 up to 296 tiles, then 16x16
 # 3-D: 8x4x4 up to 148 tiles, then 8x8x8
 SIZES = [(2, 1, 1), (29, 1, 1), (30, 1, 1), (31, 1, 1), (61, 1, 1), (4440, 1, 1), (4441, 1, 1), (37296, 1, 1),
          (37297, 1, 1), (7, 9, 1), (8, 8, 1), (9, 8, 1), (96, 96, 1), (96, 104, 1), (97, 97, 1), (256, 148, 1),
