@@ -16,6 +16,11 @@ precision and size class.  A candidate is
 
 Schedules never change results (each cell is computed the same way whatever
 the tiling, order or split), only speed.
+
+An FP64 class of few items takes small tiles of its own whatever the schedule
+(batch_few_tile, hmn_kernels.cu), so a sample of few is repeated until its
+largest class follows the schedule: its candidates would otherwise all be the
+same launches, and noise would choose what larger batches run on.
 """
 from __future__ import annotations
 
@@ -28,6 +33,7 @@ import numpy as np
 TILE_VARIANTS = {0: (0, 1), 1: (2, 3), 2: (4,)}  # tile ids per kind (include/hormone_gpu.h)
 GRID_SIZES = (0, 1, 2, 4)                          # CTAs per SM; 0 = occupancy limit
 SWEEPS = (0, 1, 2)                                 # HMN_SWEEP_STATIC, _INTERLEAVED, _DYNAMIC
+FEW = {0: ((8, 4, 4), 1), 1: ((8, 8, 1), 2), 2: ((30, 1, 1), 4)}  # batch_few_tile: tile, and items per SM up to which
 DEFAULT_CACHE = os.path.join(os.path.expanduser("~"), ".cache", "hormone_b200", "autotune.json")
 
 
@@ -63,12 +69,32 @@ def _save(path, data):
         pass
 
 
+def sm_count() -> int:
+    import torch
+
+    return torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count \
+        if torch.cuda.is_available() else 0
+
+
+def copies(kind: int, sims, precision: int) -> int:
+    """How often the sample is laid into the scratch batch: once, or in FP64 as
+    often as its largest class (with a field, without) needs to have more than
+    few items."""
+    if precision != 0:
+        return 1
+    tile, per_sm = FEW[kind]
+    items = {False: 0, True: 0}
+    for cfg, _ in sims:
+        items[bool(cfg["mag_on"])] += int(np.prod([-(-n // t) for n, t in zip(cfg["n"], tile)]))
+    return per_sm * sm_count() // max(items.values()) + 1
+
+
 def time_steps(batch, steps: int) -> float:
     """Milliseconds per batch step, timed with CUDA events on the batch's stream."""
     import torch
 
     stream = torch.cuda.ExternalStream(batch.stream_ptr())
-    batch.step(1)  # builds the graph for the current schedule
+    batch.step(steps)  # makes the work list of the current schedule, and what graphs as many steps use
     batch.sync()
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     e0.record(stream)
@@ -99,6 +125,10 @@ def tune(sample: List[Tuple[dict, dict]], precision: int = 0, steps: int = 3, ca
     for kind, sims in by_kind.items():
         cells = int(np.mean([np.prod(c["n"]) for c, _ in sims]))
         key = f"k{kind}_p{precision}_s{size_class(cells)}_n{min(len(sims), 64)}"
+        times = copies(kind, sims, precision)
+        if times > 1:
+            key += f"_x{times}"
+            sims = sims * times
         if key in data and len(data[key].get("schedule", ())) == 3:
             best[kind] = tuple(data[key]["schedule"])
             continue

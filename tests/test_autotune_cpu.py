@@ -85,6 +85,29 @@ def test_two_field_cache_entries_are_tuned_again(fake, tmp_path):
     assert len(fake.made) == 2
 
 
+def test_a_sample_of_few_items_is_repeated_until_it_follows_the_schedule(fake, tmp_path, monkeypatch):
+    monkeypatch.setattr(autotune, "sm_count", lambda: 148)
+    path = tmp_path / "t.json"
+    sims = [cases.kh2d(16), cases.kh2d(24)]  # 4 + 9 tiles of 8x8 against 296
+    assert autotune.tune(sims, cache=str(path)) == {1: (3, 2, 2)}
+    assert fake.made[0].added == 2 * 23  # 23 * 13 = 299
+    # an entry that an unrepeated sample left under the plain key is not served
+    assert list(json.loads(path.read_text())) == ["k1_p0_s8_n2_x23"]
+    assert autotune.tune(sims, cache=str(path)) == {1: (3, 2, 2)} and len(fake.made) == 1
+    autotune.tune(sims, precision=1, cache=str(path))  # the mixed form always follows the schedule
+    assert fake.made[1].added == 2
+
+
+@pytest.mark.parametrize("kind,n,items", [(0, (9, 8, 8), 8), (1, (17, 8, 1), 3), (2, (61, 1, 1), 3)])
+def test_copies_end_just_past_few(monkeypatch, kind, n, items):
+    monkeypatch.setattr(autotune, "sm_count", lambda: 148)
+    tile, per_sm = autotune.FEW[kind]
+    for count in (1, 7):
+        for mags in ([True] * count, [True] * count + [False]):  # the largest class counts
+            c = autotune.copies(kind, [(dict(n=list(n), mag_on=m), None) for m in mags], 0)
+            assert c * count * items > per_sm * 148 >= (c - 1) * count * items
+
+
 def test_apply_sets_tile_grid_and_sweep():
     b = FakeBatch(0)
     autotune.apply(b, {1: (3, 4, 1), 0: (0, 0)})  # a two-field schedule means the static sweep
