@@ -157,7 +157,8 @@ class Batch:
         return out
 
     def set_schedule(self, kind: int, tile_id: int, blocks_per_sm: int = 0):
-        """kind 0 3-D / 1 2-D x-y / 2 1-D x; tile_id per include/hormone_gpu.h."""
+        """kind 0 3-D / 1 2-D x-y / 2 1-D x; tile_id per include/hormone_gpu.h.
+        FP64 classes of few items take smaller tiles of their own."""
         rc = capi.lib().hmn_batch_set_schedule(self.h, int(kind), int(tile_id), int(blocks_per_sm))
         if rc != 0:
             raise capi.HmnError(rc, "hmn_batch_set_schedule")

@@ -5,9 +5,12 @@
 // by footprint: hmn_batch_add fails with HMN_ENOMEM when the pool has no
 // room) and a descriptor in a device array.  A batch step runs, for all
 // simulations at once, the step of src/main/hormone.f90:126-147 on each
-// simulation's own clock: CFL reduction, dt with the clamps, rktype fused
-// RK stages and the time advance -- one persistent launch per phase and
-// tile kind, captured in a CUDA graph that is replayed for every step.
+// simulation's own clock.  The simulations of one tile kind and physics form a
+// class; the classes run side by side, each with one launch per RK stage and
+// one that reduces the CFL quantities of the new state (in the last stage where
+// the class has few items).  One launch for all then advances the clocks and
+// forms the next dt with its clamps, so that a step ends with what the next one
+// starts from.  A list of simulations that lasts is stepped by CUDA graphs.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -112,7 +112,9 @@ __device__ __forceinline__ double recip_core(double b) {
   return __fma_rn(y, e, y);
 }
 
-// RN(1/b); sets bad where b is out of range or has an all-ones significand
+// RN(1/b) of either sign; sets bad where b is out of range or has an all-ones
+// significand.  (The kernels pair div_rn below with reciprocals formed on the
+// host; tests/div_check.cu checks it with these.)
 __device__ __forceinline__ double recip_rn(double b, bool& bad) {
   bad = bad || !fin_range(b) || ones_significand(b);
   return recip_core(b);

@@ -12,14 +12,17 @@
 // its output so the next stage reads primitives without dividing again.
 //
 // One RK stage (hydro.f90:35-41: boundarycondition -> numflux -> source ->
-// rungekutta) is ONE launch of stage_kernel.  A CTA owns a tile of 256 cells:
+// rungekutta) is ONE launch of stage_kernel (3-D Cartesian grids without
+// passive scalars: of the march, hmn_march.cu).  A CTA owns a tile of 30 to 512
+// cells, by the grid's dimension and size:
 //   1. it stages the primitives of the tile and of two cells beyond each face
 //      of the tile (a cross-shaped region, no corners) into shared memory,
 //      forming ghost cells from the boundary codes on the fly
 //      (boundarycondition.f90, codes 0-3 and the ghost energy of :222-243);
 //   2. per solved axis it computes the limited slopes (interpolation.f90),
-//      the HLLD face fluxes (numflux.f90 + hlldflux.f90) and adds the flux
-//      divergence of its cell to registers;
+//      the face fluxes (numflux.f90 + hlldflux.f90; without a field from the
+//      two star states of the contact wave) and adds the flux divergence of its
+//      cell to registers;
 //   3. it applies the RK combination (rungekutta.f90:35-59) with the gravity
 //      source (source.f90:70-85) and writes U and P of the new state.
 // Slopes and fluxes never leave the SM.
@@ -543,7 +546,8 @@ using F3D = Tile<8, 4, 4, 192, 1>;
 using F2D = Tile<8, 8, 1, 96, 1>;
 using F1D = Tile<30, 1, 1, 32, 1>;
 
-// tile ids: 0 3-D 8x8x8 (640 threads), 1 3-D 8x8x4 (256 threads, 2 CTAs/SM),
+// tile ids: 0 3-D 8x8x8 (640 threads), 1 3-D 8x8x4 (384 threads, 2 CTAs/SM, 3
+// without a field),
 // 2 2-D 16x16, 3 2-D 32x8, 4 1-D 256.  batch_tile_kind gives the grid's
 // kind (0 3-D, 1 2-D x-y, 2 1-D x); each kind has the tile ids listed in
 // batch_tile_variants.
@@ -578,10 +582,16 @@ void batch_tile_shape(int tid, int tile[3]) {
 // The tile a class of few items takes instead of the schedule's (ids 5 to 7,
 // chosen inside a batch only): as in the persistent small-grid loop, a step of
 // small grids is a chain of phases as long as one CTA's work, so the class is
-// cut into small tiles as long as they leave an SM about one warp per
-// scheduler: `most` is that many items.  Their last RK stage also reduces the
-// CFL quantities of the state it writes, which a class that fills the GPU does
-// not, for it would pay for the reduction's arithmetic at the stage's occupancy.
+// cut into small tiles as long as those are all resident at once: `most` items,
+// 4 of 30 cells per SM (one warp per scheduler), 2 of 8x8 (three warps each) or 1
+// of 8x4x4 (six warps).  Their last RK stage also reduces the CFL quantities of the
+// state it writes, which a class that fills the GPU does not, for it would pay for
+// the reduction's arithmetic at the stage's occupancy.  us per step of one class,
+// small tiles against the schedule's (16x16, 8x8x8, 256), with a field: 1-D 900
+// cells 31.0 / 38.7 at 30 items, 33.2 / 43.2 at 450; 2-D 24^2 47.8 / 79.3 at 144
+// items, 51.8 / 78.0 at 225, 78.9 / 77.9 at 320 (64^2); 3-D 12^3 65.8 / 122.1 at 144,
+// 122.6 / 121.7 at 216.  Without a field, and in 1-D, the small tiles stay ahead up to
+// about twice these limits, which other classes' CTAs beside them may need.
 int batch_few_tile(int kind, int nsm, int* most) {
   *most = (kind == 0 ? 1 : (kind == 1 ? 2 : 4)) * nsm;
   return 5 + kind;

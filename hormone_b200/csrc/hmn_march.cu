@@ -23,9 +23,10 @@
 // Why a march: a z slope and a z face are computed once per cell instead of
 // 10/8 and 9/8 times for an 8x8x8 tile; each plane is staged once per column
 // tile instead of a cross-shaped 8x8x8 region (1,280 cells per 512); and the
-// shared memory (108 KB: three 16x8 planes with their x-y halo, x-y slopes
-// and fluxes of one plane, the z slopes and fluxes of one plane) lets two
-// CTAs share an SM, so one CTA's barrier waits overlap the other's work.
+// shared memory (112 KB with a field: three 16x8 planes with their x-y halo,
+// x-y slopes and fluxes of one plane, the z slopes and fluxes of one plane)
+// lets two CTAs share an SM, so one CTA's barrier waits overlap the other's
+// work; without a field it is 64 KB, and three do.
 // The z quantities of a column stay with the thread that owns it: its z
 // slopes and z flux wait in shared memory slots that only this thread uses,
 // and it applies the z flux difference in phase 3.
@@ -34,9 +35,9 @@
 // and about 190 of them per cell are IEEE divisions, most sharing a
 // denominator with others (per face, 35 quotients have 11 denominators).
 // Slopes, faces and the primitive recovery form them with FastDiv
-// (hmn_div.cuh): one correctly rounded reciprocal per denominator, then a
-// branch-free two-step correction per quotient, which yields the IEEE
-// quotient bit for bit; where an operand lies outside the range in which
+// (hmn_div.cuh): one correctly rounded reciprocal per denominator, then one
+// branch-free correction per quotient, which yields the IEEE quotient bit for
+// bit; where an operand lies outside the range in which
 // that holds, the slope, face or cell is recomputed with IEEE division.
 #include <cuda_runtime.h>
 
@@ -415,13 +416,16 @@ __global__ void __launch_bounds__(MT::NT, (MAG ? MT::MINB : MT::MINBH))
 
 // 16x8 columns with 128 more threads; the owners take x-y items too, so
 // every thread has one to two items per phase.  Without a field the phases
-// are short and wait on latency and barriers, and the layout takes 66 KB
-// instead of 111: three CTAs per SM at 80 registers (the 160^3 polytrope, 8
+// are short and wait on latency and barriers, and the layout takes 64.3 KB
+// instead of 111.6: three CTAs per SM at 80 registers (the 160^3 polytrope, 8
 // steps with copies: 56.1 -> 51.1 ms).
-using MT168 = March<16, 8, 128, 2, 3>;
+using MT = March<16, 8, 128, 2, 3>;
+// an SM's 228 KB, 1 KB of them taken by the system for each CTA
+static_assert(MT::MINB * (sizeof(MarchSmem<MT, true>) + 1024) <= 228 * 1024, "CTAs per SM with a field");
+static_assert(MT::MINBH * (sizeof(MarchSmem<MT, false>) + 1024) <= 228 * 1024, "CTAs per SM without a field");
 
-template <bool MAG, bool GLM, int LIM, bool PUSH, class MT>
-cudaError_t launch_mt(const GridDev& G, const StageArgs& A, int LZ, int ntx, int nty, int nch, cudaStream_t st) {
+template <bool MAG, bool GLM, int LIM, bool PUSH>
+cudaError_t launch_t(const GridDev& G, const StageArgs& A, int LZ, int ntx, int nty, int nch, cudaStream_t st) {
   constexpr int smem = (int)sizeof(MarchSmem<MT, MAG>);
   static bool attr = false;
   if (!attr) {
@@ -435,11 +439,6 @@ cudaError_t launch_mt(const GridDev& G, const StageArgs& A, int LZ, int ntx, int
   }
   march_stage_kernel<MAG, GLM, LIM, MT, PUSH><<<ntx * nty * nch, MT::NT, smem, st>>>(G, A, LZ, ntx, nty);
   return cudaGetLastError();
-}
-
-template <bool MAG, bool GLM, int LIM, bool PUSH>
-cudaError_t launch_t(const GridDev& G, const StageArgs& A, int LZ, int ntx, int nty, int nch, cudaStream_t st) {
-  return launch_mt<MAG, GLM, LIM, PUSH, MT168>(G, A, LZ, ntx, nty, nch, st);
 }
 
 template <bool MAG, bool GLM, bool PUSH>
@@ -478,8 +477,8 @@ bool march_enabled() {
 }
 
 void march_chunks(const int n[3], int* lz, int* ntx, int* nty, int* nch) {
-  *ntx = (n[0] + MT168::TX - 1) / MT168::TX;
-  *nty = (n[1] + MT168::TY - 1) / MT168::TY;
+  *ntx = (n[0] + MT::TX - 1) / MT::TX;
+  *nty = (n[1] + MT::TY - 1) / MT::TY;
   // z chunks: about twelve CTAs per SM in all (six waves of two), each chunk at least 16 planes
   const long long cols = (long long)(*ntx) * (*nty);
   long long want = (12LL * sm_count() + cols - 1) / cols;

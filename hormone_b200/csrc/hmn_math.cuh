@@ -241,8 +241,16 @@ __device__ __forceinline__ void hlld(T f[9], T cfl, T cfr, T v1l, T v1r, T v2l, 
 // face instead of 11, 35 and 9.  A result equals that of hlld as long as no
 // dropped term is NaN or infinite: the policy refuses operands for which one
 // might be (densities outside [2^-150, 2^200), velocities from 2^150 on, wave
-// distances outside [2^-200, 2^200), a star density that is not positive).  Where sm = -0, hlld takes the state between
-// the Alfven waves, but every flux then has the factor sm.
+// distances outside [2^-200, 2^200), a star density that is not positive).  Where
+// sm = -0, hlld takes the state between the Alfven waves, but every flux then has
+// the factor sm.
+//
+// T = float (the mixed form): there the compiler contracts both solvers, and not
+// alike, so the bits differ from hlld<float> while the error does not grow.
+// Against 64 bits, over 4 M faces in each of 15 ranges (jumps of 0 to e^2 in density
+// and pressure, Mach 0.1 to 5), the rms error of every flux is 0.95 to 1.00 of
+// hlld<float>'s (2e-8 to 6e-7 of the local scale) and the largest 0.87 to 1.10; a
+// mixed step of 160x150x140 cells takes 1.82 ms instead of 2.13.
 template <typename T, class D>
 __device__ __forceinline__ void hllc(T f[5], T csl, T csr, T v1l, T v1r, T v2l, T v2r, T v3l, T v3r, T dl, T dr, T el,
                                      T er, T ptl, T ptr, D& dvp) {

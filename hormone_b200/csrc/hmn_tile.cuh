@@ -46,15 +46,16 @@ __device__ __forceinline__ size_t cidx(const GridDev& G, int i, int j, int k) {
   return (size_t)i + (size_t)G.n[0] * ((size_t)j + (size_t)G.n[1] * (size_t)k);
 }
 
-// Compile-time description of a tile: TX x TY x TZ cells (256 in all) and a
-// halo of two cells beyond each face of every axis with extent > 1.
+// Compile-time description of a tile: TX x TY x TZ cells (30 to 512 in all)
+// and a halo of two cells beyond each face of every axis with extent > 1.
 template <int TX_, int TY_, int TZ_, int NT_ = 256, int MINB_ = 2, int SP_ = 0, int MINBH_ = MINB_>
 struct Tile {
   static constexpr int TX = TX_, TY = TY_, TZ = TZ_;
   static constexpr int SP = SP_;      // passive scalars the shared-memory layout has room for
   // threads per CTA: at least the tile's cell count, and best the size of the
   // largest per-axis slope box, so that every phase of an axis pass takes one
-  // round (16x16 -> 288, 256 -> 288, 32x8 -> 320, 8x8x4 -> 384, 8x8x8 -> 640)
+  // round (30 -> 32, 126 -> 128, 256 -> 288, 8x8 -> 96, 16x16 -> 288, 32x8 ->
+  // 320, 8x4x4 -> 192, 8x8x4 -> 384, 8x8x8 -> 640)
   static constexpr int NT = NT_;
   // resident CTAs per SM the register budget is sized for, with and without a field
   static constexpr int MINB = MINB_, MINBH = MINBH_;

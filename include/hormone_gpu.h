@@ -343,7 +343,15 @@ int hmn_batch_download(hmn_batch* b, int sim, double* u, double* const prim[9]);
  * (tile_id 0 = 8x8x8 or 1 = 8x8x4 for 3-D, 2 = 16x16 or 3 = 32x8 for
  * 2-D, 4 = 256 for 1-D) and the persistent-grid size of the stage
  * launches in CTAs per SM (0: the occupancy limit).  The autotuner sets
- * it; results do not depend on it. */
+ * it; results do not depend on it.
+ *
+ * The schedule and the sweep below hold for the mixed form and for FP64
+ * classes (the listed simulations of one kind, with a field or without)
+ * that fill the GPU.  An FP64 class that would leave most of it idle takes
+ * smaller tiles, all resident at once, and leaves the schedule aside: up to
+ * one tile of 8x4x4 cells per SM in 3-D, two of 8x8 in 2-D, four of 30 in
+ * 1-D.  Which of the two holds is decided whenever the list of simulations
+ * changes. */
 int hmn_batch_set_schedule(hmn_batch* b, int kind, int tile_id, int blocks_per_sm);
 
 /* Sweep schedule of one grid kind's stage launches: the order of the
@@ -354,7 +362,8 @@ int hmn_batch_set_schedule(hmn_batch* b, int kind, int tile_id, int blocks_per_s
  *                          static split
  *   HMN_SWEEP_DYNAMIC      the largest simulations first; CTAs take the
  *                          next item from a shared counter
- * The autotuner sets it; results do not depend on it. */
+ * The autotuner sets it; results do not depend on it.  It holds where the
+ * schedule does. */
 #define HMN_SWEEP_STATIC 0
 #define HMN_SWEEP_INTERLEAVED 1
 #define HMN_SWEEP_DYNAMIC 2
