@@ -79,7 +79,9 @@ def test_schedule_does_not_change_results(precision):
     """Tile shape, grid size and sweep (static, interleaved, dynamic) give
     the same bits, also when the schedule changes between steps (the work
     list and graph are rebuilt) and over many replays of one graph (the
-    dynamic queue resets itself after every launch)."""
+    dynamic queue resets itself after every launch).  In FP64 these classes
+    have few items and keep to their own tiles; test_gpu_batch_schedules.py has
+    the ones that follow the schedule."""
     sims = mix()[:5]  # 2-D, 3-D and 1-D kinds
     outs = []
     for i, sched in enumerate(SCHEDULES):
